@@ -1,4 +1,6 @@
 // Class dispatch entry used by the host code (kept in a CUDA translation unit).
+#include <algorithm>
+
 #include "eri_launch.cuh"
 #include "host_internal.h"
 
@@ -7,7 +9,7 @@ namespace cintx {
 cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const QuartetRec* recs, int nrec,
                          const ShellPair* pairs, const PrimPair* prims, double* out, OutStrides st,
                          double expcutoff, const RysTable& rys, cudaStream_t stream, bool fp32,
-                         double prim_eps, int variant, const double* rootbuf, const long long* rootbase) {
+                         double prim_eps, int variant, const double* rootbuf, const long long* rootbase, int nsplit) {
   LaunchArgs a;
   a.recs = recs;
   a.nrec = nrec;
@@ -24,7 +26,22 @@ cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const Quartet
   a.variant = variant;
   a.rootbuf = rootbuf;
   a.rootbase = rootbase;
+  a.nsplit = nsplit;
   return dispatch_eri(li, lj, lk, ll, sph, a);
+}
+
+PrimSplit prim_split(int li, int lj, int lk, int ll, double work, long long nrec, double pmax) {
+  PrimSplit r;
+  const int s = pick_threads(li, lj, lk, ll, variant_acc(0));
+  const int most = split_max(s);
+  if (most <= 1 || nrec <= 0) return r;
+  const double resident = (double)device_sm_count() * 4 * (128 / s);
+  const double share = std::max(work / resident, s == 1 ? 16.0 : 4.0);
+  if (pmax < 2 * share) return r;
+  r.ns = 2;
+  while (r.ns < most && r.ns * share < pmax) r.ns *= 2;
+  r.pmin = (double)nrec * r.ns <= 2 * resident ? 0 : 2 * share;
+  return r;
 }
 
 static_assert(kNumVariants == kLaunchVariants, "variant count differs between kernel and host headers");

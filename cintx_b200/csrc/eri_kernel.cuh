@@ -228,6 +228,31 @@ __device__ __forceinline__ void quartet_sync(int group) {
   }
 }
 
+// Barrier of a split team: `threads` consecutive threads (a power of two) that share one quartet, team
+// number `team` of the block.  Teams of at most a warp meet by warp mask, a team that fills the block
+// at the block barrier, teams of 64 threads (two per block) at named barriers 1 and 2; those ids are
+// free there, because the groups of such teams have at most 32 lanes (group_sync by warp mask).
+__device__ __forceinline__ void team_sync(int threads, int team) {
+  if (threads <= 32) {
+    const unsigned base = threadIdx.x & 31u & ~(unsigned)(threads - 1);
+    __syncwarp(threads == 32 ? 0xffffffffu : (((1u << threads) - 1u) << base));
+  } else if (threads == (int)blockDim.x) {
+    __syncthreads();
+  } else {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(threads) : "memory");
+  }
+}
+
+// How a team of ns members (a power of two) shares the nij x nkl primitive quartets of its quartet:
+// members form an la x (ns / la) grid over (a, b), member m taking a = m % la, + la, ... and
+// b = m / la, + ns / la, ...  la is at most 8 while there are b's to share, so that the members of one
+// b leave the screened a loop (sorted by decreasing bound) within a few iterations of each other.
+__device__ __forceinline__ int split_la(int ns, int nij, int nkl) {
+  int la = ns;
+  while (la > 1 && (la > 8 || (la >> 1) >= nij) && ns / la < nkl) la >>= 1;
+  return la;
+}
+
 // e[j][a] = C(j, a) x^(j - a) for a <= j <= N (zero above the diagonal), by Pascal's rule
 // e[j][a] = e[j-1][a-1] + x e[j-1][a]: the binomial weights of the horizontal transfer come out of
 // multiply-adds on registers, with no integer binomial evaluated in the unrolled loops.
@@ -462,16 +487,17 @@ __device__ __forceinline__ void prim_loop_one_lane(const ShellPair& pij, const S
                                                    const PrimPair* __restrict__ prims, const RysTable& rys,
                                                    const double* tab, double expcutoff, double prim_eps,
                                                    const double* __restrict__ rb, const LaneTuples<SH>& lt,
-                                                   double (&acc)[SH::TPT][SH::NFI]) {
+                                                   double (&acc)[SH::TPT][SH::NFI], int a0 = 0, int da = 1,
+                                                   int b0 = 0, int db = 1) {
   constexpr int NR = SH::NR, GSZ = SH::GSZ, NFI = SH::NFI, TPT = SH::TPT;
   constexpr bool SSSS = LI + LJ + LK + LL == 0;
-  for (int b = 0; b < pkl.nprim; ++b) {
+  for (int b = b0; b < pkl.nprim; b += db) {
     const PrimPair pk = prims[pkl.prim_off + b];
     const double qcx = pk.px - pkl.ax, qcy = pk.py - pkl.ay, qcz = pk.pz - pkl.az;
     // primitive Schwarz screening: (ij) pairs are sorted by q, so stop at the first one whose
     // bound q_ij * q_kl < prim_eps (prim_eps == 0 gives NaN or 0 here: never stops)
     const double qthr = prim_eps / pk.q;
-    for (int a = 0; a < pij.nprim; ++a) {
+    for (int a = a0; a < pij.nprim; a += da) {
       const PrimPair pi = prims[pij.prim_off + a];
       if (pi.q < qthr) break;
       if (pi.cce + pk.cce > expcutoff) continue;  // CINT2e_loop eijcutoff (cint2e.c:700-712)
@@ -558,14 +584,19 @@ __device__ __forceinline__ void prim_loop_one_lane(const ShellPair& pij, const S
   }
 }
 
+// SPLIT: a quartet is shared by a team of nsplit groups (a power of two, nsplit * S <= BLOCK, one warp at
+// most for S == 1), each evaluating its share of the primitive quartets (split_la); their partial
+// blocks are added before the j, k and l transform stages, which all lanes of the team run.  It is the
+// shape of launches whose longest quartet would otherwise run on long after the others (prim_split).
 template <int LI, int LJ, int LK, int LL, bool SPH, class R = double, int ACC = 24, int REGS = 128,
-          bool SLICE = false, bool ROLL = false, int PASSES = 1>
+          bool SLICE = false, bool ROLL = false, int PASSES = 1, bool SPLIT = false>
 __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>::BLOCK,
                                   EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>::MINB)
     eri4c_kernel(const QuartetRec* __restrict__ recs, int nrec, const ShellPair* __restrict__ pairs,
                  const PrimPair* __restrict__ prims, double* __restrict__ out, OutStrides st,
                  double expcutoff, const __grid_constant__ RysTable rys, double* __restrict__ gscratch,
-                 double prim_eps, const double* __restrict__ rootbuf, const long long* __restrict__ rootbase) {
+                 double prim_eps, const double* __restrict__ rootbuf, const long long* __restrict__ rootbase,
+                 int nsplit) {
   using SH = EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>;
   constexpr int S = SH::S, NR = SH::NR, GSZ = SH::GSZ, NFI = SH::NFI, TPT = SH::TPT;
   constexpr bool FP64 = std::is_same<R, double>::value;
@@ -584,6 +615,8 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
   static_assert(SLICE || S == 1 || (SH::B_GROUP % 16 == 0 && SH::B_ROOTS % 16 == 0 && SH::TABLE_DOUBLES % 2 == 0 &&
                                     (SH::NI % 2 != 0 || SH::GSZ % 2 == 0)),
                 "16-byte loads of the I arrays need 16-byte aligned group regions and tables");
+  static_assert(!SPLIT || (!SLICE && FP64 && !SH::GLOBAL_BUF && S < 128 && SH::BLOCK == 128 && SH::Q * S == 128),
+                "split teams: FP64 shapes with several groups in a block of 128 threads");
   const int group = SLICE ? (int)(threadIdx.x / (32 * LN)) * 32 + (int)(threadIdx.x & 31) : (int)threadIdx.x / S;
   const int lane = SLICE ? (int)(threadIdx.x / 32) % LN : (int)threadIdx.x % S;
   char* sgb = reinterpret_cast<char*>(smem + SH::TABLE_DOUBLES) + group * SH::B_GROUP;
@@ -607,8 +640,11 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
 
   // q = blockIdx.x * Q + group; in sliced shapes every thread of a set runs the trip count of the
   // set's first quartet (the set shares barriers) and lanes past the end only take part in them
-  const int qfirst = SLICE ? (int)blockIdx.x * SH::Q + (group & ~31) : (int)blockIdx.x * SH::Q + group;
-  for (int qb = qfirst; qb < nrec; qb += gridDim.x * SH::Q) {
+  const int ns = SPLIT ? nsplit : 1;  // groups sharing a quartet
+  const int team = SPLIT ? group / ns : group, sub = SPLIT ? group % ns : 0;
+  const int per_block = SPLIT ? SH::Q / ns : SH::Q;  // quartets a block holds
+  const int qfirst = SLICE ? (int)blockIdx.x * SH::Q + (group & ~31) : (int)blockIdx.x * per_block + team;
+  for (int qb = qfirst; qb < nrec; qb += gridDim.x * per_block) {
     const int qv = SLICE ? qb + (group & 31) : qb;
     const bool live = !SLICE || qv < nrec;
     const int q = live ? qv : nrec - 1;
@@ -623,9 +659,26 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
 #pragma unroll
       for (int f = 0; f < NFI; ++f) acc[k][f] = 0.0;
 
+    int a0 = 0, da = 1, b0 = 0, db = 1;  // this group's share of the primitive quartets
+    if constexpr (SPLIT) {
+      da = split_la(ns, pij.nprim, pkl.nprim);
+      db = ns / da;
+      a0 = sub % da;
+      b0 = sub / da;
+    }
     if constexpr (S == 1) {
       prim_loop_one_lane<LI, LJ, LK, LL, SH, R>(pij, pkl, prims, rys, SH::STAGE_TABLE ? smem : nullptr, expcutoff,
-                                                prim_eps, rb, lt, acc);
+                                                prim_eps, rb, lt, acc, a0, da, b0, db);
+      if constexpr (SPLIT) {  // the team's partial blocks: every lane of the team ends with the sum
+        const unsigned tmask =
+            ns == 32 ? 0xffffffffu : (((1u << ns) - 1u) << (threadIdx.x & 31u & ~(unsigned)(ns - 1)));
+        for (int o = ns >> 1; o > 0; o >>= 1) {
+#pragma unroll
+          for (int k = 0; k < TPT; ++k)
+#pragma unroll
+            for (int f = 0; f < NFI; ++f) acc[k][f] += __shfl_xor_sync(tmask, acc[k][f], o);
+        }
+      }
     } else if constexpr (SLICE) {
       // each lane runs the register path for its own tuple slice (lane + S*k)
       static_loop(std::make_integer_sequence<int, S>{}, [&](auto j) {
@@ -657,14 +710,14 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
         }
       });
     } else
-    for (int b = 0; b < pkl.nprim; ++b) {
+    for (int b = b0; b < pkl.nprim; b += db) {
       const PrimPair pk = prims[pkl.prim_off + b];
-      if (b + 1 < pkl.nprim) prefetch_prim(prims + pkl.prim_off + b + 1);
+      if (b + db < pkl.nprim) prefetch_prim(prims + pkl.prim_off + b + db);
       const double qcx = pk.px - pkl.ax, qcy = pk.py - pkl.ay, qcz = pk.pz - pkl.az;
       const double qthr = prim_eps / pk.q;  // as in prim_loop_one_lane
-      for (int a = 0; a < pij.nprim; ++a) {
+      for (int a = a0; a < pij.nprim; a += da) {
         const PrimPair pi = prims[pij.prim_off + a];
-        if (a + 1 < pij.nprim) prefetch_prim(prims + pij.prim_off + a + 1);
+        if (a + da < pij.nprim) prefetch_prim(prims + pij.prim_off + a + da);
         if (pi.q < qthr) break;
         if (pi.cce + pk.cce > expcutoff) continue;  // CINT2e_loop eijcutoff (cint2e.c:700-712)
         const double aij = pi.aij, akl = pk.aij;
@@ -797,11 +850,16 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
                   }
                 }
               }
-              obase[mi * st.s0 + mj * st.s1 + mk * st.s2 + ml * st.s3] = v;
+              if (!SPLIT || sub == 0) obase[mi * st.s0 + mj * st.s1 + mk * st.s2 + ml * st.s3] = v;
             }
     } else {
       double* bufA = SH::GLOBAL_BUF ? gscratch + (size_t)blockIdx.x * SH::GBUF_PER_BLOCK : sg;
-      double* bufB = bufA + SH::SM_BUFA;
+      // lanes of the j, k and l stages: the group's, or those of the whole team
+      const int tl = SPLIT ? sub * S + lane : lane, tn = SPLIT ? ns * S : LN;
+      auto block_sync = [&]() {
+        if constexpr (SPLIT) team_sync(tn, team);
+        else quartet_sync<LN, SLICE, SH::BLOCK>(group);
+      };
       // stage i in registers -> bufA[mi + MI * t], t = fj + NFJ*(fk + NFK*fl) (two-pass sliced
       // shapes stored it after each pass)
 #pragma unroll
@@ -820,12 +878,24 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
           }
         }
       }
-      quartet_sync<LN, SLICE, SH::BLOCK>(group);
+      block_sync();
+      if constexpr (SPLIT) {  // add the groups' partial blocks into the first group's buffer
+        constexpr int GD = SH::B_GROUP / 8;
+        double* first = sg - (size_t)sub * GD;
+        for (int e = tl; e < SH::MI * SH::NTUP; e += tn) {
+          double v = first[e];
+          for (int g = 1; g < ns; ++g) v += first[(size_t)g * GD + e];
+          first[e] = v;
+        }
+        bufA = first;
+        block_sync();
+      }
+      double* bufB = bufA + SH::SM_BUFA;
       // stage j: bufA[mi + MI*(fj + NFJ*(fk + NFK*fl))] -> bufB[mi + MI*(mj + MJ*(fk + NFK*fl))]
       const double* cur = bufA;
       if constexpr (SPH && LJ >= 2) {
         constexpr int n = SH::MI * SH::MJ * SH::NFK * SH::NFL;
-        for (int o = lane; o < n; o += LN) {
+        for (int o = tl; o < n; o += tn) {
           const int mi = o % SH::MI;
           const int mj = (o / SH::MI) % SH::MJ;
           const int rest = o / (SH::MI * SH::MJ);
@@ -834,14 +904,14 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
           for (int z = 0; z < row.nnz; ++z) v += row.c[z] * bufA[mi + SH::MI * (row.f[z] + SH::NFJ * rest)];
           bufB[o] = v;
         }
-        quartet_sync<LN, SLICE, SH::BLOCK>(group);
+        block_sync();
         cur = bufB;
       }
       // stage k: cur[mi + MI*(mj + MJ*(fk + NFK*fl))] -> nxt[mi + MI*(mj + MJ*(mk + MK*fl))]
       if constexpr (SPH && LK >= 2) {
         double* nxt = (cur == bufA) ? bufB : bufA;
         constexpr int n = SH::MI * SH::MJ * SH::MK * SH::NFL;
-        for (int o = lane; o < n; o += LN) {
+        for (int o = tl; o < n; o += tn) {
           const int mij = o % (SH::MI * SH::MJ);
           const int mk = (o / (SH::MI * SH::MJ)) % SH::MK;
           const int fl = o / (SH::MI * SH::MJ * SH::MK);
@@ -851,14 +921,14 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
             v += row.c[z] * cur[mij + SH::MI * SH::MJ * (row.f[z] + SH::NFK * fl)];
           nxt[o] = v;
         }
-        quartet_sync<LN, SLICE, SH::BLOCK>(group);
+        block_sync();
         cur = nxt;
       }
       // stage l + store: cur[mijk + MIJK*fl] -> out
       {
         constexpr int n = SH::NOUT;
         constexpr int MIJK = SH::MI * SH::MJ * SH::MK;
-        for (int o = lane; o < n; o += LN) {
+        for (int o = tl; o < n; o += tn) {
           const int mi = o % SH::MI;
           const int mj = (o / SH::MI) % SH::MJ;
           const int mk = (o / (SH::MI * SH::MJ)) % SH::MK;
@@ -875,7 +945,7 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
           if (live) obase[mi * st.s0 + mj * st.s1 + mk * st.s2 + ml * st.s3] = v;
         }
       }
-      quartet_sync<LN, SLICE, SH::BLOCK>(group);
+      block_sync();
     }
   }
 }

@@ -23,6 +23,7 @@ struct LaunchArgs {
   int variant = 0;      // launch-shape variant (spherical FP64 classes; see variant_acc)
   const double* rootbuf = nullptr;     // precomputed roots [record's base + (b*npij + a)*2*NR]
   const long long* rootbase = nullptr;  // per record of this launch: its base in rootbuf
+  int nsplit = 1;       // groups sharing one quartet's primitive quartets (power of two; prim_split)
 };
 
 // Device scratch for classes whose transform buffers live in global memory: returns a buffer
@@ -37,16 +38,19 @@ __host__ __device__ constexpr bool class_valid(int li, int lj, int lk, int ll) {
 
 int device_sm_count();
 
+// Largest number of groups of s lanes that can share a quartet (0: the shape has no split form).
+__host__ __device__ constexpr int split_max(int s) { return s == 1 ? 32 : (s < 128 ? 128 / s : 0); }
+
 }  // namespace cintx
 #include "eri_splitcoop.cuh"
 namespace cintx {
 
 template <int LI, int LJ, int LK, int LL, bool SPH, class R = double, int ACC = 24, int REGS = 128,
-          bool SLICE = false, bool ROLL = false, int PASSES = 1>
+          bool SLICE = false, bool ROLL = false, int PASSES = 1, bool SPLIT = false>
 cudaError_t launch_eri(const LaunchArgs& a) {
   using SH = EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>;
   if (a.query) return SH::GLOBAL_BUF ? cudaErrorNotSupported : cudaSuccess;
-  auto kern = eri4c_kernel<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>;
+  auto kern = eri4c_kernel<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES, SPLIT>;
   static int attr_done[64];
   int dev = 0;
   cudaGetDevice(&dev);
@@ -56,7 +60,11 @@ cudaError_t launch_eri(const LaunchArgs& a) {
     attr_done[dev] = 1;
   }
   if (a.nrec <= 0) return cudaSuccess;
-  long long blocks = ((long long)a.nrec + SH::Q - 1) / SH::Q;
+  // a team of nsplit groups must be a power of two inside one block (one warp for one-lane groups)
+  if (SPLIT && (a.nsplit < 1 || a.nsplit > split_max(SH::S) || (a.nsplit & (a.nsplit - 1)) != 0))
+    return cudaErrorInvalidValue;
+  const int per_block = SPLIT ? SH::Q / a.nsplit : SH::Q;
+  long long blocks = ((long long)a.nrec + per_block - 1) / per_block;
   long long cap = a.max_blocks > 0 ? a.max_blocks : (long long)device_sm_count() * 32;
   if (blocks > cap) blocks = cap;
   double* scratch = nullptr;
@@ -67,7 +75,7 @@ cudaError_t launch_eri(const LaunchArgs& a) {
   }
   kern<<<(unsigned)blocks, SH::BLOCK, SH::SMEM_BYTES, a.stream>>>(a.recs, a.nrec, a.pairs, a.prims, a.out,
                                                                    a.st, a.expcutoff, a.rys, scratch, a.prim_eps,
-                                                                   a.rootbuf, a.rootbase);
+                                                                   a.rootbuf, a.rootbase, a.nsplit);
   return cudaGetLastError();
 }
 
@@ -96,7 +104,15 @@ cudaError_t dispatch_lij(int lk, int ll, bool sph, const LaunchArgs& a) {
           constexpr int s2 = pick_threads(LI, LJ, k, l, variant_acc(2));
           // only shapes that differ from the default are instantiated (if constexpr)
           bool done = false;
-          if (a.fp32) {
+          if constexpr (split_max(s0) > 1) {
+            if (!a.fp32 && a.nsplit > 1) {
+              err = sph ? launch_eri<LI, LJ, k, l, true, double, 24, 128, false, false, 1, true>(a)
+                        : launch_eri<LI, LJ, k, l, false, double, 24, 128, false, false, 1, true>(a);
+              done = true;
+            }
+          }
+          if (done) {
+          } else if (a.fp32) {
             err = sph ? launch_eri<LI, LJ, k, l, true, float>(a) : cudaErrorInvalidValue;
             done = true;
           } else if (!sph) {

@@ -668,6 +668,7 @@ static int eval_call(int family, bool sph, double* out, int* dims, int* shls, in
   std::vector<QuartetRec> recs;
   std::vector<PrimPair> allprims;
   bool any = false;
+  double pwork = 0, pmax = 0;  // primitive quartets: all, and of the largest contraction tuple
   // enumerate contraction tuples
   int nc0 = nctr[0], nc1 = nctr[1], nc2 = nctr[2], nc3 = nctr[3];
   for (int c3 = 0; c3 < nc3; ++c3)
@@ -682,6 +683,9 @@ static int eval_call(int family, bool sph, double* out, int* dims, int* shls, in
           build_pair(*B, vs[ori.src[2]], vs[ori.src[3]], cutoff, p2);
           const bool pe = p1.prims.empty() || p2.prims.empty() || (p1.min_cce + p2.min_cce > cutoff);
           if (!pe) any = true;
+          const double np = (double)p1.prims.size() * (double)p2.prims.size();
+          pwork += np;
+          pmax = std::max(pmax, np);
           QuartetRec q;
           q.pij = (int)pairs.size();
           p1.sp.prim_off = (int)allprims.size();
@@ -734,7 +738,8 @@ static int eval_call(int family, bool sph, double* out, int* dims, int* shls, in
   for (int c = 0; c < 4; ++c) *sv[c] = axstride[ori.src[c]];
   cudaError_t e = launch_class(ori.li, ori.lj, ori.lk, ori.ll, sph, (const QuartetRec*)(d + off_recs), (int)recs.size(),
                                (const ShellPair*)(d + off_pairs), (const PrimPair*)(d + off_prims),
-                               (double*)(d + off_out), st, cutoff, ds->rys, ts->stream);
+                               (double*)(d + off_out), st, cutoff, ds->rys, ts->stream, false, 0.0, 0, nullptr, nullptr,
+                               prim_split(ori.li, ori.lj, ori.lk, ori.ll, pwork, (long long)recs.size(), pmax).ns);
   if (e != cudaSuccess) {
     set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("kernel launch failed: ") + cudaGetErrorString(e));
     return 0;

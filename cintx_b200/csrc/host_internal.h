@@ -166,7 +166,21 @@ cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const Quartet
                          const ShellPair* pairs, const PrimPair* prims, double* out, OutStrides st,
                          double expcutoff, const RysTable& rys, cudaStream_t stream, bool fp32 = false,
                          double prim_eps = 0.0, int variant = 0, const double* rootbuf = nullptr,
-                         const long long* rootbase = nullptr);
+                         const long long* rootbase = nullptr, int nsplit = 1);
+// Which quartets of one launch share their primitive quartets over several lane groups.  A group's
+// lanes walk a quartet's primitive quartets one after another, so a launch lasts at least as long as
+// its largest quartet (4096 primitive quartets of two contracted s pairs: 1.2 ms on one lane).  `work`
+// is the launch's primitive quartets, `pmax` its largest quartet's: where that is over twice the
+// share that a resident group (4 blocks of 128 threads per SM) has when the work is spread evenly,
+// quartets of at least pmin primitive quartets run on ns groups each (ns = 1: none do; pmin = 0: the
+// whole launch, which then still fits the resident groups twice).  A share under 16 primitive
+// quartets on one lane (4 on a wider group) is not split further: adding up the partial blocks would
+// cost as much.
+struct PrimSplit {
+  int ns = 1;
+  double pmin = 0;
+};
+PrimSplit prim_split(int li, int lj, int lk, int ll, double work, long long nrec, double pmax);
 // Learned Rys roots (rysnet.cu) of order n at count device points: out[p*2n + f], status[p]
 // (0 refined, 1 table fallback, 2 closed form), asynchronous on stream.
 cudaError_t rys_learned_eval(const float* d_params, const RysTable& rys, int n, const double* d_x, long long count,

@@ -70,6 +70,7 @@ struct Segment {
   bool fp32 = false;       // FP32 recurrences (mixed-precision plans)
   double prim_eps = 0;     // primitive Schwarz threshold (tuned plans)
   int variant = 0;         // launch shape chosen by cintx_plan_autotune (0: default)
+  int nsplit = 1;          // groups sharing each quartet's primitive quartets (prim_split); > 1: default shape
   bool swap = false;       // screened: the tile's records are (col, row) pairs
 };
 
@@ -245,6 +246,7 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
     std::vector<QuartetRec> recs;
     std::vector<int> tuples;
     double flops = 0;
+    double work = 0, pmax = 0;  // primitive quartets: all, and of the largest record
   };
   PhaseLog plog("explicit plan");
   // 1. requested shells and block sizes (serial; the first bad shell index ends the plan)
@@ -399,6 +401,8 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
                                 flops_c2s(k.li, k.lj, k.lk, k.ll, p->sph);
               P.flops += fq;
               last->flops += fq;
+              last->work += (double)npq;
+              last->pmax = std::max(last->pmax, (double)npq);
             }
     }
   };
@@ -450,6 +454,7 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
   Chunk ch;
   long long rec0 = 0;
   std::vector<std::pair<const Group*, long long>> copies;  // (part group, first record)
+  std::vector<std::pair<size_t, double>> heavy;            // segments split in two: (index, pmin)
   for (auto& kv : joined) {
     Segment sg;
     sg.li = kv.first.li;
@@ -465,11 +470,17 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
     sg.nrec = 0;
     sg.out_off = 0;
     sg.flops = 0;
+    double work = 0, pmax = 0;
     for (const Group* g : kv.second) {
       copies.emplace_back(g, rec0 + sg.nrec);
       sg.nrec += (long long)g->recs.size();
       sg.flops += g->flops;
+      work += g->work;
+      pmax = std::max(pmax, g->pmax);
     }
+    const PrimSplit ps = prim_split(sg.li, sg.lj, sg.lk, sg.ll, work, sg.nrec, pmax);
+    sg.nsplit = ps.ns;
+    if (ps.ns > 1 && ps.pmin > 0) heavy.emplace_back(ch.segs.size(), ps.pmin);
     ch.segs.push_back(sg);
     rec0 += sg.nrec;
   }
@@ -489,6 +500,27 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
     for (int t = 1; t < nc; ++t) th.emplace_back(place);
     place();
     for (auto& x : th) x.join();
+  }
+  // a class whose large quartets share lane groups: those records first, the others in a segment of
+  // their own (the tuples keep the order they are reported in)
+  for (size_t h = heavy.size(); h-- > 0;) {
+    Segment& big = ch.segs[heavy[h].first];
+    const double pmin = heavy[h].second;
+    auto npq = [&](const QuartetRec& r) { return (double)o->pair_nprim[r.pij] * (double)o->pair_nprim[r.pkl]; };
+    auto r0 = p->h_recs.begin() + big.rec0, r1 = r0 + big.nrec;
+    auto mid = std::stable_partition(r0, r1, [&](const QuartetRec& r) { return npq(r) >= pmin; });
+    if (mid == r0 || mid == r1) continue;
+    double wb = 0, ws = 0;
+    for (auto r = r0; r != mid; ++r) wb += npq(*r);
+    for (auto r = mid; r != r1; ++r) ws += npq(*r);
+    Segment rest = big;
+    rest.nsplit = 1;
+    rest.rec0 = big.rec0 + (mid - r0);
+    rest.nrec = r1 - mid;
+    rest.flops = big.flops * ws / (wb + ws);
+    big.nrec = mid - r0;
+    big.flops -= rest.flops;
+    ch.segs.insert(ch.segs.begin() + heavy[h].first + 1, rest);
   }
   ch.out_size = off;
   ch.nrec = rec0;
@@ -551,7 +583,8 @@ static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStr
     const bool rb = p->d_rootbuf && sg.tile == -1;  // learned roots: explicit plans only
     cudaError_t e = launch_class(sg.li, sg.lj, sg.lk, sg.ll, p->sph, recs + r0, nr, o->d_pairs, o->d_prims,
                                  out_dev + sg.out_off, sg.st, sg.expcutoff, ds->rys, stream, sg.fp32, sg.prim_eps,
-                                 sg.variant, rb ? p->d_rootbuf : nullptr, rb ? p->d_rootbase + sg.rec0 + r0 : nullptr);
+                                 sg.variant, rb ? p->d_rootbuf : nullptr, rb ? p->d_rootbase + sg.rec0 + r0 : nullptr,
+                                 sg.nsplit);
     if (e != cudaSuccess) {
       set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("kernel launch failed: ") + cudaGetErrorString(e));
       return CINTX_STATUS_EXECUTION_FAILED;
@@ -1124,7 +1157,10 @@ int cintx_plan_autotune(CintxPlan* p, int64_t chunk, double* out_dev, void* stre
       const Segment& sg = p->chunks[c].segs[i];
       const auto key = std::make_tuple(sg.li, sg.lj, sg.lk, sg.ll, (int)sg.fp32);
       auto it = target.find(key);
-      if (it == target.end() || (chunk < 0 && p->chunks[it->second.first].segs[it->second.second].nrec < sg.nrec))
+      const Segment* cur = it == target.end() ? nullptr : &p->chunks[it->second.first].segs[it->second.second];
+      // segments of split quartets run the default shape: timed only where a class has no other
+      if (!cur || (cur->nsplit > 1 && sg.nsplit == 1) ||
+          (chunk < 0 && (cur->nsplit > 1) == (sg.nsplit > 1) && cur->nrec < sg.nrec))
         target[key] = std::make_pair(c, i);
     }
   cudaEvent_t e0, e1;
@@ -1146,7 +1182,7 @@ int cintx_plan_autotune(CintxPlan* p, int64_t chunk, double* out_dev, void* stre
     std::vector<int> lanes_seen;
     double best_ms = 1e300;
     int best_v = 0;
-    for (int v = 0; v < kLaunchVariants && !rc; ++v) {
+    for (int v = 0; v < (sg0.nsplit > 1 ? 1 : kLaunchVariants) && !rc; ++v) {
       const int shape = variant_shape(sg0.li, sg0.lj, sg0.lk, sg0.ll, p->sph, sg0.fp32, v);
       if (std::find(lanes_seen.begin(), lanes_seen.end(), shape) != lanes_seen.end()) continue;
       lanes_seen.push_back(shape);
@@ -1604,8 +1640,7 @@ int compute_prim_schwarz(Opt* o) {
 // Contracted Schwarz factors Q_ij = sqrt(max |(ij|ij)|) of every stored pair, from its spherical
 // diagonal block: the class kernels evaluate the blocks into the thread's device scratch (classes
 // (la lb|la lb), batches of at most 2^25 doubles), block_absmax_sqrt_kernel reduces each block to
-// its factor, and only the factors come back to the host.  Same kernels, launch shapes and records
-// as an explicit plan of the tuples (a b a b), so the factors are those of that plan bit for bit.
+// its factor, and only the factors come back to the host.
 // np < 0: every stored pair; else the first np.
 int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
   if (np < 0 || np > o->npairs) np = o->npairs;  // the first np stored pairs (all by default)
@@ -1617,6 +1652,21 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
   std::map<std::pair<int, int>, std::vector<int>> cls;  // (la, lb) -> pair ids
   for (int id = 0; id < np; ++id)
     if (o->pair_nprim[id] > 0) cls[std::make_pair(o->pair_la[id], o->pair_lb[id])].push_back(id);
+  // per class, the pairs whose diagonal quartets share lane groups (prim_split) first
+  std::map<std::pair<int, int>, PrimSplit> split;
+  auto diag_np = [&](int id) { return (double)o->pair_nprim[id] * (double)o->pair_nprim[id]; };
+  for (auto& kv : cls) {
+    double work = 0, pmax = 0;
+    for (int id : kv.second) {
+      work += diag_np(id);
+      pmax = std::max(pmax, diag_np(id));
+    }
+    const PrimSplit ps =
+        prim_split(kv.first.first, kv.first.second, kv.first.first, kv.first.second, work, (long long)kv.second.size(), pmax);
+    if (ps.ns > 1)
+      std::stable_partition(kv.second.begin(), kv.second.end(), [&](int id) { return diag_np(id) >= ps.pmin; });
+    split[kv.first] = ps;
+  }
   const long long cap = 1LL << 25;  // doubles of diagonal blocks per batch
   std::vector<QuartetRec> recs;
   std::vector<long long> len;
@@ -1641,10 +1691,18 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
         for (size_t g = 0; g < seg_cls.size() && ok; ++g) {
           const int la = seg_cls[g].first, lb = seg_cls[g].second;
           const OutStrides st = canonical_strides(la, lb, la, true);
-          for (long long q0 = r0; q0 < seg_end[g] && ok; q0 += 1LL << 30) {
-            const int nr = (int)std::min<long long>(seg_end[g] - q0, 1LL << 30);
-            ok = launch_class(la, lb, la, lb, true, d_recs + q0, nr, o->d_pairs, o->d_prims, d_out, st, ecut,
-                              ds->rys, ts->stream, false, 0.0, 0, nullptr, nullptr) == cudaSuccess;
+          // the batch's records of this class: split ones [r0, rs), the others [rs, end); a batch holds
+          // far fewer than 2^30 records
+          const PrimSplit& ps = split[seg_cls[g]];
+          long long rs = r0;
+          if (ps.ns > 1)
+            while (rs < seg_end[g] && diag_np(ids[rs]) >= ps.pmin) ++rs;
+          for (int part = 0; part < 2 && ok; ++part) {
+            const long long q0 = part ? rs : r0, q1 = part ? seg_end[g] : rs;
+            if (q1 <= q0) continue;
+            ok = launch_class(la, lb, la, lb, true, d_recs + q0, (int)(q1 - q0), o->d_pairs, o->d_prims, d_out, st,
+                              ecut, ds->rys, ts->stream, false, 0.0, 0, nullptr, nullptr, part ? 1 : ps.ns) ==
+                 cudaSuccess;
             ts->launches++;
           }
           r0 = seg_end[g];
@@ -1752,8 +1810,9 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
   // flops: per tile class
   {
     // recompute nprim-weighted flops per tile
-    for (const Tile& t : p->tiles) {
-      const long long tp = t.nprimq >= 0 ? t.nprimq : tile_prim_quartets(t, o);
+    for (Tile& t : p->tiles) {
+      if (t.nprimq < 0) t.nprimq = tile_prim_quartets(t, o);
+      const long long tp = t.nprimq;
       nprimq += tp;
       const long long nq = t.row_prefix.back();
       flops += tp * flops_per_prim_quartet(t.li, t.lj, t.lk, t.ll) + nq * flops_c2s(t.li, t.lj, t.lk, t.ll, p->sph);
@@ -1920,7 +1979,8 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
     }
     ch.segs.clear();
     long long rec = 0;
-    for (auto& mem : members) {
+    // one class's pieces, all in one segment, or its large quartets (prim_split) in one and the rest in another
+    auto add_segment = [&](const std::vector<int>& mem, int nsplit) {
       const Segment& p0 = ch.pieces[mem[0]];
       Segment m;
       m.li = p0.li;
@@ -1933,6 +1993,7 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
       m.fp32 = p0.fp32;
       m.prim_eps = p0.prim_eps;
       m.swap = p0.swap;
+      m.nsplit = nsplit;
       m.rec0 = rec;
       m.out_off = 0;
       m.range0 = (int)p->ranges.size();
@@ -1958,6 +2019,33 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
       m.nranges = (int)p->ranges.size() - m.range0;
       rec += m.nrec;
       ch.segs.push_back(m);
+    };
+    // mean primitive quartets of a piece's quartets (a tile's pairs have counts within a half octave
+    // each, or for 3-centre tiles up to their shells' products)
+    auto piece_np = [&](int i) {
+      const Tile& t = p->tiles[ch.pieces[i].tile];
+      return (double)t.nprimq / (double)t.row_prefix.back();
+    };
+    for (auto& mem : members) {
+      const Segment& p0 = ch.pieces[mem[0]];
+      double work = 0, pmax = 0;
+      long long nq = 0;
+      for (int i : mem) {
+        const long long n = ch.pieces[i].t1 - ch.pieces[i].t0;
+        nq += n;
+        work += n * piece_np(i);
+        pmax = std::max(pmax, piece_np(i));
+      }
+      PrimSplit ps;
+      if (!p0.fp32) ps = prim_split(p0.li, p0.lj, p0.lk, p0.ll, work, nq, pmax);
+      if (ps.ns == 1 || ps.pmin <= 0) {
+        add_segment(mem, ps.ns);
+        continue;
+      }
+      std::vector<int> large, rest;
+      for (int i : mem) (piece_np(i) >= ps.pmin ? large : rest).push_back(i);
+      if (!large.empty()) add_segment(large, ps.ns);
+      if (!rest.empty()) add_segment(rest, 1);
     }
   }
   if (ok && !p->ranges.empty()) {

@@ -1,0 +1,54 @@
+"""Quartets whose primitive quartets are shared by several lane groups (prim_split): single-block
+calls and short lists of contracted shells, where the split is widest, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from cintx_b200 import molecules as M
+
+pytestmark = pytest.mark.gpu
+
+
+
+def contracted(ls, nprims, seed):
+    """Three atoms, each with one shell per (l, nprim)."""
+    rng = M.SplitMix64(seed)
+    coords = [[0.0, 0.0, 0.0], [0.9, -0.7, 1.1], [-1.3, 0.4, 0.6]]
+    return M.build_molecule("contracted", coords, [[M.make_shell(rng, l, n) for l, n in zip(ls, nprims)] for _ in coords])
+
+
+def agree(got, ref):
+    d = np.abs(got - ref)
+    assert np.all((d <= 1e-12) | (d <= 1e-10 * np.abs(ref))), d.max()
+
+
+@pytest.mark.parametrize("sph", [True, False])
+@pytest.mark.parametrize("nij,nkl", [(1, 17), (17, 1), (3, 7), (8, 8), (13, 17)])
+def test_single_block_calls(sph, nij, nkl):
+    import cintx_b200 as cx
+    from oracle import Restatement
+    for la, lb, lc, ld in [(0, 0, 0, 0), (1, 0, 0, 0), (2, 0, 1, 0), (1, 1, 1, 0), (2, 1, 1, 1), (3, 0, 2, 0), (2, 2, 2, 1)]:
+        mol = contracted([la, lb, lc, ld], [nij, 1 if nij > 8 else nij, nkl, 1 if nkl > 8 else nkl], 5 + la)
+        q = np.array([[0, 5, 10, 3]], dtype=np.int32)  # one shell of each kind, over the three atoms
+        ref, _ = Restatement().int2e_batch(q, mol, sph=sph)
+        f = cx.int2e_sph if sph else cx.int2e_cart
+        agree(f(q[0], mol.atm, mol.bas, mol.env)[0], ref)
+
+
+@pytest.mark.parametrize("sph", [True, False])
+def test_lists_mix_split_and_whole_quartets(sph):
+    """A list long enough that only its contracted quartets are split."""
+    import cintx_b200 as cx
+    import torch
+    from oracle import Restatement
+    mol = contracted([0, 0, 0, 1, 1, 2], [13, 1, 8, 3, 1, 1], 9)
+    rng = np.random.default_rng(3)
+    q = rng.integers(0, mol.nbas, size=(6000, 4)).astype(np.int32)
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+        plan = cx.Plan.shells(opt, cx.INT2E, q, sph=sph)
+        out = torch.full((plan.stats.nintegrals,), np.nan, dtype=torch.float64, device="cuda")
+        plan.execute(out.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        plan.close()
+    ref, _ = Restatement().int2e_batch(q, mol, sph=sph)
+    agree(got, ref)
