@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -594,6 +595,106 @@ static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStr
   return CINTX_STATUS_SUCCESS;
 }
 
+// Side streams and events of one forked chunk.  Sets are kept per device in a free list: a call takes
+// one while it queues its launches and gives it back, so there are as many as threads ever queued at
+// once, and no call records an event that another one is still to wait for.
+constexpr int kSideStreams = 7;
+struct SideStreams {
+  cudaStream_t s[kSideStreams];
+  cudaEvent_t fork, join[kSideStreams];
+};
+static std::mutex g_side_mu;
+static std::map<int, std::vector<SideStreams*>> g_side;
+
+static SideStreams* take_side_streams(int dev) {
+  {
+    std::lock_guard<std::mutex> lk(g_side_mu);
+    std::vector<SideStreams*>& v = g_side[dev];
+    if (!v.empty()) {
+      SideStreams* r = v.back();
+      v.pop_back();
+      return r;
+    }
+  }
+  SideStreams* r = new SideStreams();
+  bool ok = cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming) == cudaSuccess;
+  for (int i = 0; i < kSideStreams && ok; ++i)
+    ok = cudaStreamCreateWithFlags(&r->s[i], cudaStreamNonBlocking) == cudaSuccess &&
+         cudaEventCreateWithFlags(&r->join[i], cudaEventDisableTiming) == cudaSuccess;
+  if (ok) return r;
+  if (r->fork) cudaEventDestroy(r->fork);
+  for (int i = 0; i < kSideStreams; ++i) {
+    if (r->s[i]) cudaStreamDestroy(r->s[i]);
+    if (r->join[i]) cudaEventDestroy(r->join[i]);
+  }
+  delete r;
+  cudaGetLastError();  // the caller runs on one stream instead
+  return nullptr;
+}
+static void give_side_streams(int dev, SideStreams* r) {
+  std::lock_guard<std::mutex> lk(g_side_mu);
+  g_side[dev].push_back(r);
+}
+
+// Runs one chunk's segments on `stream`, each followed by after(segment, its stream) where given.
+// Segments are independent (disjoint records and output blocks), and most launches of a molecule of
+// some ten atoms fill a fraction of the chip for some ten microseconds, so they are spread over the
+// caller's stream and side streams that start after its earlier work and that it waits for, largest
+// segments first.  Classes that keep their transform buffers in the thread's one device scratch stay
+// on the caller's stream, in order.  A stream under capture is used alone, as before.
+static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_t stream, DeviceState* ds,
+                     ThreadScratch* ts, const std::function<int(const Segment&, cudaStream_t)>& after) {
+  int rc = CINTX_STATUS_SUCCESS;
+  const int n = (int)ch.segs.size();
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  SideStreams* side = nullptr;
+  double total = 0;
+  for (const Segment& sg : ch.segs) total += sg.flops;
+  if (n > 1 && total < kForkFlops * n) {
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) cudaGetLastError();  // used alone, as it is
+    else if (cap == cudaStreamCaptureStatusNone) side = take_side_streams(ds->dev);
+  }
+  if (!side) {
+    for (const Segment& sg : ch.segs) {
+      if ((rc = run_segment(p, sg, out_dev, stream, ds, ts))) return rc;
+      if (after && (rc = after(sg, stream))) return rc;
+    }
+    return CINTX_STATUS_SUCCESS;
+  }
+  const int nside = std::min(kSideStreams, n - 1);
+  std::vector<int> idx(n);
+  std::iota(idx.begin(), idx.end(), 0);
+  std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return ch.segs[a].flops > ch.segs[b].flops; });
+  double load[kSideStreams + 1] = {0};
+  bool used[kSideStreams + 1] = {false};
+  cudaError_t e = cudaEventRecord(side->fork, stream);
+  for (int i : idx) {
+    const Segment& sg = ch.segs[i];
+    int b = 0;
+    if (!class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant))
+      b = (int)(std::min_element(load, load + nside + 1) - load);
+    // a launch costs some microseconds however small its work
+    load[b] += sg.flops + 3e7;
+    cudaStream_t st = b == 0 ? stream : side->s[b - 1];
+    if (b > 0 && !used[b] && e == cudaSuccess) e = cudaStreamWaitEvent(st, side->fork, 0);
+    used[b] = true;
+    if (e != cudaSuccess) break;
+    if ((rc = run_segment(p, sg, out_dev, st, ds, ts)) || (after && (rc = after(sg, st)))) break;
+  }
+  for (int b = 1; b <= nside; ++b)
+    if (used[b]) {
+      const cudaError_t r1 = cudaEventRecord(side->join[b - 1], side->s[b - 1]);
+      const cudaError_t r2 = cudaStreamWaitEvent(stream, side->join[b - 1], 0);
+      if (e == cudaSuccess) e = r1 != cudaSuccess ? r1 : r2;
+    }
+  give_side_streams(ds->dev, side);
+  if (!rc && e != cudaSuccess) {
+    set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("side streams failed: ") + cudaGetErrorString(e));
+    rc = CINTX_STATUS_EXECUTION_FAILED;
+  }
+  return rc;
+}
+
 static int exec_prepare(CintxPlan* p, double* out_dev, void* stream_, cudaStream_t* stream, DeviceState** ds,
                         ThreadScratch** ts) {
   if (!p || !out_dev) {
@@ -620,8 +721,7 @@ int cintx_plan_execute(CintxPlan* p, int64_t chunk, double* out_dev, void* strea
   }
   const int64_t c0 = chunk < 0 ? 0 : chunk, c1 = chunk < 0 ? (int64_t)p->chunks.size() : chunk + 1;
   for (int64_t c = c0; c < c1; ++c)
-    for (const Segment& sg : p->chunks[c].segs)
-      if ((rc = run_segment(p, sg, out_dev, stream, ds, ts))) return rc;
+    if ((rc = run_chunk(p, p->chunks[c], out_dev, stream, ds, ts, nullptr))) return rc;
   return CINTX_STATUS_SUCCESS;
 }
 
@@ -943,18 +1043,21 @@ int cintx_plan_execute_ao(CintxPlan* p, int aosym, double* eri, int64_t len, voi
     return CINTX_STATUS_ALLOCATION_FAILED;
   }
   cudaMemsetAsync(eri, 0, sizeof(double) * need, stream);  // quartets below the cutoff stay 0
-  for (int64_t c = 0; c < (int64_t)p->chunks.size(); ++c) {
-    int rc = cintx_plan_execute(p, c, p->d_stage, stream);
-    if (rc) return rc;
-    const cudaError_t e = aosym == 8 ? launch_scatter_s8(p->d_recs, p->chunks[c].nrec, p->d_psh, p->d_aoloc,
-                                                         p->d_stage, eri, stream)
-                                     : launch_scatter_ao(p->d_recs, p->chunks[c].nrec, p->d_psh, p->d_aoloc,
-                                                         p->d_stage, eri, aosym, nao, stream);
-    if (e != cudaSuccess) {
-      set_error(CINTX_STATUS_EXECUTION_FAILED, "scatter launch failed");
-      return CINTX_STATUS_EXECUTION_FAILED;
-    }
-  }
+  DeviceState* ds;
+  ThreadScratch* ts;
+  int rc;
+  if ((rc = device_state(&ds)) || (rc = thread_scratch(&ts, 0, 0))) return rc;
+  auto scatter = [&](const Segment& sg, cudaStream_t st) -> int {
+    const QuartetRec* recs = p->d_recs + sg.rec0;
+    const cudaError_t e =
+        aosym == 8 ? launch_scatter_s8(recs, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, eri, st)
+                   : launch_scatter_ao(recs, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, eri, aosym, nao, st);
+    if (e == cudaSuccess) return CINTX_STATUS_SUCCESS;
+    set_error(CINTX_STATUS_EXECUTION_FAILED, "scatter launch failed");
+    return CINTX_STATUS_EXECUTION_FAILED;
+  };
+  for (const Chunk& ch : p->chunks)
+    if ((rc = run_chunk(p, ch, p->d_stage, stream, ds, ts, scatter))) return rc;
   return CINTX_STATUS_SUCCESS;
 }
 
@@ -1001,22 +1104,23 @@ int cintx_plan_jk(CintxPlan* p, const double* dm, int nao, double* vj, double* v
   double* A = vj ? p->d_jkacc : nullptr;
   double* Bk = vk ? p->d_jkacc + (size_t)nao * nao : nullptr;
   cudaMemsetAsync(p->d_jkacc, 0, sizeof(double) * acc, stream);
-  // each chunk: the sweep's kernels into the ring, then its contraction (same stream, so the
-  // next chunk's record generation waits for the contraction to have read the records)
-  for (int64_t c = 0; c < (int64_t)p->chunks.size(); ++c) {
-    int rc = cintx_plan_execute(p, c, p->d_stage, stream);
-    if (rc) return rc;
-    // one contraction launch per class segment: small blocks one thread per quartet, others a warp
-    for (const Segment& sg : p->chunks[c].segs) {
-      const int n = nsph_or_cart(sg.li, p->sph) * nsph_or_cart(sg.lj, p->sph) * nsph_or_cart(sg.lk, p->sph) *
-                    nsph_or_cart(sg.ll, p->sph);
-      if (launch_jk_contract(p->d_recs + sg.rec0, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, dm, nao, A, Bk, stream,
-                             n) != cudaSuccess) {
-        set_error(CINTX_STATUS_EXECUTION_FAILED, "J/K contraction launch failed");
-        return CINTX_STATUS_EXECUTION_FAILED;
-      }
-    }
-  }
+  // each chunk: every class segment's kernels into the ring, then its contraction (small blocks one
+  // thread per quartet, others a warp); the next chunk's record generation waits for all of them
+  DeviceState* ds;
+  ThreadScratch* ts;
+  int rc;
+  if ((rc = device_state(&ds)) || (rc = thread_scratch(&ts, 0, 0))) return rc;
+  auto contract = [&](const Segment& sg, cudaStream_t st) -> int {
+    const int n = nsph_or_cart(sg.li, p->sph) * nsph_or_cart(sg.lj, p->sph) * nsph_or_cart(sg.lk, p->sph) *
+                  nsph_or_cart(sg.ll, p->sph);
+    if (launch_jk_contract(p->d_recs + sg.rec0, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, dm, nao, A, Bk, st, n) ==
+        cudaSuccess)
+      return CINTX_STATUS_SUCCESS;
+    set_error(CINTX_STATUS_EXECUTION_FAILED, "J/K contraction launch failed");
+    return CINTX_STATUS_EXECUTION_FAILED;
+  };
+  for (const Chunk& ch : p->chunks)
+    if ((rc = run_chunk(p, ch, p->d_stage, stream, ds, ts, contract))) return rc;
   if ((vj && launch_symmetrize(A, vj, nao, stream) != cudaSuccess) ||
       (vk && launch_symmetrize(Bk, vk, nao, stream) != cudaSuccess)) {
     set_error(CINTX_STATUS_EXECUTION_FAILED, "J/K symmetrisation launch failed");
