@@ -641,7 +641,12 @@ static void give_side_streams(int dev, SideStreams* r) {
 // some ten atoms fill a fraction of the chip for some ten microseconds, so they are spread over the
 // caller's stream and side streams that start after its earlier work and that it waits for, largest
 // segments first.  Classes that keep their transform buffers in the thread's one device scratch stay
-// on the caller's stream, in order.  A stream under capture is used alone, as before.
+// on the caller's stream, in order.  A stream under capture is used alone, and so is the caller's
+// stream for chunks whose segments average over kForkFlops: those launches fill the chip by
+// themselves, and a segment's J/K contraction finds less of its blocks in L2 when others run beside it
+// (J/K of 120 s/p/d/f atoms, 2e10 flops a segment: 309 ms in order, 315 forked; all quartets of 3 atoms
+// 1.37 ms in order, 0.29 forked; 24-atom s/p/d/f sweep, 3e8 a segment, 13.0 and 6.9 ms).
+constexpr double kForkFlops = 4e9;
 static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_t stream, DeviceState* ds,
                      ThreadScratch* ts, const std::function<int(const Segment&, cudaStream_t)>& after) {
   int rc = CINTX_STATUS_SUCCESS;
