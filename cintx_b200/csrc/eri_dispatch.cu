@@ -30,18 +30,21 @@ cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const Quartet
   return dispatch_eri(li, lj, lk, ll, sph, a);
 }
 
-PrimSplit prim_split(int li, int lj, int lk, int ll, double work, long long nrec, double pmax) {
+PrimSplit prim_split(int lanes, int most, double resident, double work, long long nrec, double pmax) {
   PrimSplit r;
-  const int s = pick_threads(li, lj, lk, ll, variant_acc(0));
-  const int most = split_max(s);
   if (most <= 1 || nrec <= 0) return r;
-  const double resident = (double)device_sm_count() * 4 * (128 / s);
-  const double share = std::max(work / resident, s == 1 ? 16.0 : 4.0);
+  const double share = std::max(work / resident, lanes == 1 ? 16.0 : 4.0);
   if (pmax < 2 * share) return r;
   r.ns = 2;
   while (r.ns < most && r.ns * share < pmax) r.ns *= 2;
   r.pmin = (double)nrec * r.ns <= 2 * resident ? 0 : 2 * share;
   return r;
+}
+
+PrimSplit prim_split(int li, int lj, int lk, int ll, double work, long long nrec, double pmax) {
+  const int s = pick_threads(li, lj, lk, ll, variant_acc(0));
+  if (split_max(s) <= 1) return PrimSplit();
+  return prim_split(s, split_max(s), (double)device_sm_count() * 4 * (128 / s), work, nrec, pmax);
 }
 
 static_assert(kNumVariants == kLaunchVariants, "variant count differs between kernel and host headers");

@@ -47,6 +47,43 @@ cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2
                               const double* out, double* eri, int mode, long long nao, cudaStream_t stream);
 }
 
+namespace cintx {
+
+static std::mutex g_side_mu;
+static std::map<int, std::vector<SideStreams*>> g_side;
+
+SideStreams* take_side_streams(int dev) {
+  {
+    std::lock_guard<std::mutex> lk(g_side_mu);
+    std::vector<SideStreams*>& v = g_side[dev];
+    if (!v.empty()) {
+      SideStreams* r = v.back();
+      v.pop_back();
+      return r;
+    }
+  }
+  SideStreams* r = new SideStreams();
+  bool ok = cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming) == cudaSuccess;
+  for (int i = 0; i < kSideStreams && ok; ++i)
+    ok = cudaStreamCreateWithFlags(&r->s[i], cudaStreamNonBlocking) == cudaSuccess &&
+         cudaEventCreateWithFlags(&r->join[i], cudaEventDisableTiming) == cudaSuccess;
+  if (ok) return r;
+  if (r->fork) cudaEventDestroy(r->fork);
+  for (int i = 0; i < kSideStreams; ++i) {
+    if (r->s[i]) cudaStreamDestroy(r->s[i]);
+    if (r->join[i]) cudaEventDestroy(r->join[i]);
+  }
+  delete r;
+  cudaGetLastError();  // the caller runs on one stream instead
+  return nullptr;
+}
+void give_side_streams(int dev, SideStreams* r) {
+  std::lock_guard<std::mutex> lk(g_side_mu);
+  g_side[dev].push_back(r);
+}
+
+}  // namespace cintx
+
 using namespace cintx;
 
 namespace {
@@ -595,47 +632,6 @@ static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStr
   return CINTX_STATUS_SUCCESS;
 }
 
-// Side streams and events of one forked chunk.  Sets are kept per device in a free list: a call takes
-// one while it queues its launches and gives it back, so there are as many as threads ever queued at
-// once, and no call records an event that another one is still to wait for.
-constexpr int kSideStreams = 7;
-struct SideStreams {
-  cudaStream_t s[kSideStreams];
-  cudaEvent_t fork, join[kSideStreams];
-};
-static std::mutex g_side_mu;
-static std::map<int, std::vector<SideStreams*>> g_side;
-
-static SideStreams* take_side_streams(int dev) {
-  {
-    std::lock_guard<std::mutex> lk(g_side_mu);
-    std::vector<SideStreams*>& v = g_side[dev];
-    if (!v.empty()) {
-      SideStreams* r = v.back();
-      v.pop_back();
-      return r;
-    }
-  }
-  SideStreams* r = new SideStreams();
-  bool ok = cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming) == cudaSuccess;
-  for (int i = 0; i < kSideStreams && ok; ++i)
-    ok = cudaStreamCreateWithFlags(&r->s[i], cudaStreamNonBlocking) == cudaSuccess &&
-         cudaEventCreateWithFlags(&r->join[i], cudaEventDisableTiming) == cudaSuccess;
-  if (ok) return r;
-  if (r->fork) cudaEventDestroy(r->fork);
-  for (int i = 0; i < kSideStreams; ++i) {
-    if (r->s[i]) cudaStreamDestroy(r->s[i]);
-    if (r->join[i]) cudaEventDestroy(r->join[i]);
-  }
-  delete r;
-  cudaGetLastError();  // the caller runs on one stream instead
-  return nullptr;
-}
-static void give_side_streams(int dev, SideStreams* r) {
-  std::lock_guard<std::mutex> lk(g_side_mu);
-  g_side[dev].push_back(r);
-}
-
 // Runs one chunk's segments on `stream`, each followed by after(segment, its stream) where given.
 // Segments are independent (disjoint records and output blocks), and most launches of a molecule of
 // some ten atoms fill a fraction of the chip for some ten microseconds, so they are spread over the
@@ -666,32 +662,19 @@ static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_
     }
     return CINTX_STATUS_SUCCESS;
   }
-  const int nside = std::min(kSideStreams, n - 1);
   std::vector<int> idx(n);
   std::iota(idx.begin(), idx.end(), 0);
   std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return ch.segs[a].flops > ch.segs[b].flops; });
-  double load[kSideStreams + 1] = {0};
-  bool used[kSideStreams + 1] = {false};
-  cudaError_t e = cudaEventRecord(side->fork, stream);
+  Fork fork(stream, side, n - 1);
   for (int i : idx) {
     const Segment& sg = ch.segs[i];
-    int b = 0;
-    if (!class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant))
-      b = (int)(std::min_element(load, load + nside + 1) - load);
     // a launch costs some microseconds however small its work
-    load[b] += sg.flops + 3e7;
-    cudaStream_t st = b == 0 ? stream : side->s[b - 1];
-    if (b > 0 && !used[b] && e == cudaSuccess) e = cudaStreamWaitEvent(st, side->fork, 0);
-    used[b] = true;
-    if (e != cudaSuccess) break;
+    cudaStream_t st =
+        fork.next(sg.flops + 3e7, class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant));
+    if (fork.error() != cudaSuccess) break;
     if ((rc = run_segment(p, sg, out_dev, st, ds, ts)) || (after && (rc = after(sg, st)))) break;
   }
-  for (int b = 1; b <= nside; ++b)
-    if (used[b]) {
-      const cudaError_t r1 = cudaEventRecord(side->join[b - 1], side->s[b - 1]);
-      const cudaError_t r2 = cudaStreamWaitEvent(stream, side->join[b - 1], 0);
-      if (e == cudaSuccess) e = r1 != cudaSuccess ? r1 : r2;
-    }
+  const cudaError_t e = fork.join();
   give_side_streams(ds->dev, side);
   if (!rc && e != cudaSuccess) {
     set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("side streams failed: ") + cudaGetErrorString(e));
@@ -1109,8 +1092,8 @@ int cintx_plan_jk(CintxPlan* p, const double* dm, int nao, double* vj, double* v
   double* A = vj ? p->d_jkacc : nullptr;
   double* Bk = vk ? p->d_jkacc + (size_t)nao * nao : nullptr;
   cudaMemsetAsync(p->d_jkacc, 0, sizeof(double) * acc, stream);
-  // each chunk: every class segment's kernels into the ring, then its contraction (small blocks one
-  // thread per quartet, others a warp); the next chunk's record generation waits for all of them
+  // each chunk: every class segment's kernels into the ring, then its contraction; the next chunk's
+  // record generation waits for all of them
   DeviceState* ds;
   ThreadScratch* ts;
   int rc;

@@ -66,7 +66,11 @@ struct Ip1Work {
              std::tie(o.li, o.lj, o.lk, o.ll, o.s0, o.s1, o.s2, o.s3, o.blk);
     }
   };
-  std::map<Key, std::vector<QuartetRec>> groups;
+  struct Group {
+    std::vector<QuartetRec> recs;
+    double work = 0, pmax = 0;  // primitive quartets: all, and of the largest record
+  };
+  std::map<Key, Group> groups;
   std::vector<double> pair_min_cce;  // per pair: smallest screening exponent of its primitive pairs
   long long out_doubles = 0;  // all components of all blocks
   bool any = false;           // some primitive survived screening (libcint's return value)
@@ -116,7 +120,7 @@ int ip1_build(const Basis& B, int nsh, const int* shls, int64_t n, bool sph, boo
     kfirst.emplace(key, f);
     return f;
   };
-  std::vector<QuartetRec>* last = nullptr;  // consecutive tuples mostly share a group
+  Ip1Work::Group* last = nullptr;  // consecutive tuples mostly share a group
   Ip1Work::Key last_key{};
   long long off = 0;
   for (int64_t q = 0; q < n; ++q) {
@@ -171,7 +175,10 @@ int ip1_build(const Basis& B, int nsh, const int* shls, int64_t n, bool sph, boo
               last = &W.groups[k];
               last_key = k;
             }
-            last->push_back(r);
+            last->recs.push_back(r);
+            const double np = (double)W.pairs[r.pij].nprim * W.pairs[r.pkl].nprim;
+            last->work += np;
+            last->pmax = std::max(last->pmax, np);
           }
     off += 3 * st;
   }
@@ -182,7 +189,7 @@ int ip1_build(const Basis& B, int nsh, const int* shls, int64_t n, bool sph, boo
 // Device image of the work: [pairs][primitive pairs][records], 256-byte aligned parts.
 size_t ip1_image_bytes(const Ip1Work& W, size_t* o_prims, size_t* o_recs) {
   size_t nrec = 0;
-  for (auto& kv : W.groups) nrec += kv.second.size();
+  for (auto& kv : W.groups) nrec += kv.second.recs.size();
   *o_prims = (sizeof(ShellPair) * W.pairs.size() + 255) & ~(size_t)255;
   *o_recs = (*o_prims + sizeof(PrimPair) * std::max<size_t>(W.prims.size(), 1) + 255) & ~(size_t)255;
   return *o_recs + sizeof(QuartetRec) * std::max<size_t>(nrec, 1);
@@ -192,51 +199,99 @@ size_t ip1_image_bytes(const Ip1Work& W, size_t* o_prims, size_t* o_recs) {
 // `host` (kept by the caller until the stream has consumed it) and launches every class group on
 // `stream`, writing into out_dev.
 int ip1_launch(const Ip1Work& W, bool sph, int nsh, const Basis& B, char* dev, char* host, double* out_dev,
-               cudaStream_t stream, const RysTable& rys) {
+               cudaStream_t stream, const RysTable& rys, int devid, int64_t* nlaunch) {
   size_t o_prims, o_recs;
   const size_t total = ip1_image_bytes(W, &o_prims, &o_recs);
   memcpy(host, W.pairs.data(), sizeof(ShellPair) * W.pairs.size());
   if (!W.prims.empty()) memcpy(host + o_prims, W.prims.data(), sizeof(PrimPair) * W.prims.size());
+  // a class's records, those whose primitive quartets are shared by several groups (prim_split) first
+  struct Launch {
+    const Ip1Work::Key* key;
+    size_t rec0, nrec;
+    int nsplit;
+    double work;
+  };
+  std::vector<Launch> launches;
   size_t r0 = 0;
-  std::vector<std::pair<const Ip1Work::Key*, std::pair<size_t, size_t>>> launches;
   for (auto& kv : W.groups) {
-    memcpy(host + o_recs + sizeof(QuartetRec) * r0, kv.second.data(), sizeof(QuartetRec) * kv.second.size());
-    launches.push_back({&kv.first, {r0, kv.second.size()}});
-    r0 += kv.second.size();
+    const Ip1Work::Key& k = kv.first;
+    const std::vector<QuartetRec>& recs = kv.second.recs;
+    QuartetRec* dst = reinterpret_cast<QuartetRec*>(host + o_recs) + r0;
+    int shape[3];
+    Ip1Args qa{};
+    qa.shape = shape;
+    if (dispatch_ip1(k.li, k.lj, k.lk, k.ll, sph, qa) != cudaSuccess) {
+      set_error(CINTX_STATUS_EXECUTION_FAILED, "derivative class is not compiled");
+      return CINTX_STATUS_EXECUTION_FAILED;
+    }
+    // resident groups: 512 threads per SM
+    const PrimSplit ps = prim_split(shape[0], shape[1], (double)device_sm_count() * std::max(1, 512 / shape[0]),
+                                    kv.second.work, (long long)recs.size(), kv.second.pmax);
+    auto npq = [&](const QuartetRec& r) { return (double)W.pairs[r.pij].nprim * W.pairs[r.pkl].nprim; };
+    size_t nbig = ps.ns > 1 && ps.pmin <= 0 ? recs.size() : 0;
+    double wbig = nbig ? kv.second.work : 0;
+    if (ps.ns == 1 || nbig) {
+      memcpy(dst, recs.data(), sizeof(QuartetRec) * recs.size());
+    } else {
+      for (const QuartetRec& r : recs)
+        if (npq(r) >= ps.pmin) {
+          dst[nbig++] = r;
+          wbig += npq(r);
+        }
+      size_t at = nbig;
+      for (const QuartetRec& r : recs)
+        if (!(npq(r) >= ps.pmin)) dst[at++] = r;
+    }
+    const double unit = flops_per_prim_quartet(k.li + 1, k.lj, k.lk, k.ll);
+    if (nbig) launches.push_back({&k, r0, nbig, ps.ns, wbig * unit});
+    if (nbig < recs.size()) launches.push_back({&k, r0 + nbig, recs.size() - nbig, 1, (kv.second.work - wbig) * unit});
+    r0 += recs.size();
   }
+  std::stable_sort(launches.begin(), launches.end(), [](const Launch& x, const Launch& y) { return x.work > y.work; });
   cudaError_t e = cudaMemcpyAsync(dev, host, total, cudaMemcpyHostToDevice, stream);
   if (e != cudaSuccess) {
     set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("upload failed: ") + cudaGetErrorString(e));
     return CINTX_STATUS_EXECUTION_FAILED;
   }
   const double cutoff = nsh == 4 ? expcutoff_2e(B.env.data()) : expcutoff_3c(B.env.data());
-  for (auto& L : launches) {
-    const Ip1Work::Key& k = *L.first;
-    Ip1Args a;
-    a.pairs = (const ShellPair*)dev;
-    a.prims = (const PrimPair*)(dev + o_prims);
-    a.out = out_dev;
-    a.st.s0 = k.s0;
-    a.st.s1 = k.s1;
-    a.st.s2 = k.s2;
-    a.st.s3 = k.s3;
-    a.scomp = k.blk;
-    a.expcutoff = cutoff;
-    a.rys = rys;
-    a.stream = stream;
-    const size_t base = L.second.first, cnt = L.second.second;
-    for (size_t s0 = 0; s0 < cnt; s0 += (size_t)1 << 30) {
-      a.recs = (const QuartetRec*)(dev + o_recs) + base + s0;
-      a.nrec = (int)std::min<size_t>(cnt - s0, (size_t)1 << 30);
-      e = dispatch_ip1(k.li, k.lj, k.lk, k.ll, sph, a);
-      if (e != cudaSuccess) {
-        set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("derivative kernel launch failed: ") +
-                                                     cudaGetErrorString(e));
-        return CINTX_STATUS_EXECUTION_FAILED;
+  // the launches are independent: largest first over the stream and side streams (as plan chunks)
+  SideStreams* side = launches.size() > 1 ? take_side_streams(devid) : nullptr;
+  int rc = CINTX_STATUS_SUCCESS;
+  {
+    Fork fork(stream, side, (int)launches.size() - 1);
+    for (const Launch& L : launches) {
+      const Ip1Work::Key& k = *L.key;
+      Ip1Args a{};
+      a.pairs = (const ShellPair*)dev;
+      a.prims = (const PrimPair*)(dev + o_prims);
+      a.out = out_dev;
+      a.st.s0 = k.s0;
+      a.st.s1 = k.s1;
+      a.st.s2 = k.s2;
+      a.st.s3 = k.s3;
+      a.scomp = k.blk;
+      a.expcutoff = cutoff;
+      a.rys = rys;
+      a.nsplit = L.nsplit;
+      a.stream = fork.next(L.work + 3e7);
+      e = fork.error();
+      for (size_t s0 = 0; s0 < L.nrec && e == cudaSuccess; s0 += (size_t)1 << 30) {
+        a.recs = (const QuartetRec*)(dev + o_recs) + L.rec0 + s0;
+        a.nrec = (int)std::min<size_t>(L.nrec - s0, (size_t)1 << 30);
+        e = dispatch_ip1(k.li, k.lj, k.lk, k.ll, sph, a);
       }
+      if (e != cudaSuccess) break;
+      ++*nlaunch;
     }
+    const cudaError_t ej = fork.join();
+    if (e == cudaSuccess) e = ej;
   }
-  return CINTX_STATUS_SUCCESS;
+  if (side) give_side_streams(devid, side);
+  if (e != cudaSuccess) {
+    set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("derivative kernel launch failed: ") + cudaGetErrorString(e));
+    rc = CINTX_STATUS_EXECUTION_FAILED;
+  }
+  return rc;
 }
 
 }  // namespace
@@ -270,9 +325,10 @@ int ip1_eval(int nsh, double* out, bool to_host, const int* shls, int64_t n, boo
   char* host = (char*)ts->hbuf;
   double* dout = to_host ? (double*)(dev + image) : out;
   if (to_host) cudaMemsetAsync(dout, 0, outb, ts->stream);
-  if ((rc = ip1_launch(W, sph, nsh, B, dev, host, dout, ts->stream, ds->rys))) return rc;
+  int64_t nlaunch = 0;
+  if ((rc = ip1_launch(W, sph, nsh, B, dev, host, dout, ts->stream, ds->rys, ds->dev, &nlaunch))) return rc;
   if (to_host) cudaMemcpyAsync(out, dout, outb, cudaMemcpyDeviceToHost, ts->stream);
-  ts->launches += (int64_t)W.groups.size();
+  ts->launches += nlaunch;
   const cudaError_t e = cudaStreamSynchronize(ts->stream);
   if (e != cudaSuccess) {
     set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("device execution failed: ") + cudaGetErrorString(e));

@@ -52,3 +52,28 @@ def test_lists_mix_split_and_whole_quartets(sph):
         plan.close()
     ref, _ = Restatement().int2e_batch(q, mol, sph=sph)
     agree(got, ref)
+
+
+@pytest.mark.parametrize("nsh", [3, 4])
+@pytest.mark.parametrize("sph", [True, False])
+def test_derivatives_of_contracted_shells(nsh, sph):
+    """One derivative block per call (its primitive quartets over all lane groups) equals the same
+    block out of a list of 4000 (few or none of them split)."""
+    import cintx_b200 as cx
+    import torch
+    mol = contracted([0, 0, 1, 1, 2, 3], [13, 7, 3, 1, 1, 1], 11)
+    rng = np.random.default_rng(4)
+    t = rng.integers(0, mol.nbas, size=(4000, nsh)).astype(np.int32)
+    t[:6] = np.arange(6)[:, None] + np.array([0, 6, 12, 6])[:nsh]
+    fam = cx.INT2E if nsh == 4 else cx.INT3C2E
+    out = torch.full((cx.ip1_len(fam, t, mol.bas, sph),), np.nan, dtype=torch.float64, device="cuda")
+    off = cx.ip1_eval(fam, t, mol.atm, mol.bas, mol.env, out.data_ptr(), sph)
+    got = out.cpu().numpy()
+    assert np.isfinite(got).all()
+    f = {(4, True): cx.int2e_ip1_sph, (4, False): cx.int2e_ip1_cart, (3, True): cx.int3c2e_ip1_sph,
+         (3, False): cx.int3c2e_ip1_cart}[nsh, sph]
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:  # screened as the list is
+        for q in range(40):
+            one, _ = f(t[q], mol.atm, mol.bas, mol.env, opt=opt)
+            # equal up to the order of at most 169 x 169 primitive terms of either sign
+            assert np.allclose(one, got[off[q]:off[q] + one.size], rtol=1e-9, atol=1e-11)
