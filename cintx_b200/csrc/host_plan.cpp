@@ -39,7 +39,7 @@ cudaError_t launch_block_absmax_sqrt(const QuartetRec* recs, long long nrec, con
                                      double* q, cudaStream_t stream);
 cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
                                const double* out, const double* dm, int nao, double* A, double* B, cudaStream_t stream,
-                               int block_elems);
+                               int ni, int nj, int nk, int nl);
 cudaError_t launch_symmetrize(const double* X, double* M, int n, cudaStream_t stream);
 cudaError_t launch_scatter_s8(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
                               const double* out, double* eri, cudaStream_t stream);
@@ -1099,10 +1099,9 @@ int cintx_plan_jk(CintxPlan* p, const double* dm, int nao, double* vj, double* v
   int rc;
   if ((rc = device_state(&ds)) || (rc = thread_scratch(&ts, 0, 0))) return rc;
   auto contract = [&](const Segment& sg, cudaStream_t st) -> int {
-    const int n = nsph_or_cart(sg.li, p->sph) * nsph_or_cart(sg.lj, p->sph) * nsph_or_cart(sg.lk, p->sph) *
-                  nsph_or_cart(sg.ll, p->sph);
-    if (launch_jk_contract(p->d_recs + sg.rec0, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, dm, nao, A, Bk, st, n) ==
-        cudaSuccess)
+    if (launch_jk_contract(p->d_recs + sg.rec0, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, dm, nao, A, Bk, st,
+                           nsph_or_cart(sg.li, p->sph), nsph_or_cart(sg.lj, p->sph), nsph_or_cart(sg.lk, p->sph),
+                           nsph_or_cart(sg.ll, p->sph)) == cudaSuccess)
       return CINTX_STATUS_SUCCESS;
     set_error(CINTX_STATUS_EXECUTION_FAILED, "J/K contraction launch failed");
     return CINTX_STATUS_EXECUTION_FAILED;

@@ -6,6 +6,8 @@
 // its row by binary search and writes the record; out offsets are consecutive blocks.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.h"
 
 __global__ void gen_tile_quartets(const int* __restrict__ rows, const int* __restrict__ cols,
@@ -253,66 +255,182 @@ __global__ void scatter_ao_kernel(const QuartetRec* __restrict__ recs, long long
   }
 }
 
-// As jk_contract_kernel for small blocks (all of one class, n = ni nj nk nl <= 32 elements): one
-// thread per quartet, so the many tiny blocks ((ss|ss), (ps|ss), ...) do not idle a warp each.
-__global__ void jk_contract_small_kernel(const QuartetRec* __restrict__ recs, long long nrec,
-                                         const int2* __restrict__ psh, const int* __restrict__ aoloc,
-                                         const double* __restrict__ out, const double* __restrict__ dm, int nao,
-                                         double* __restrict__ A, double* __restrict__ B) {
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < nrec; r += (long long)gridDim.x * blockDim.x) {
-    const QuartetRec rec = recs[r];
-    const int2 ab = psh[rec.pij], cd = psh[rec.pkl];
-    const int i0 = aoloc[ab.x], j0 = aoloc[ab.y], k0 = aoloc[cd.x], l0 = aoloc[cd.y];
-    const int ni = aoloc[ab.x + 1] - i0, nj = aoloc[ab.y + 1] - j0;
-    const int nk = aoloc[cd.x + 1] - k0, nl = aoloc[cd.y + 1] - l0;
-    const double s = (ab.x == ab.y ? 0.5 : 1.0) * (cd.x == cd.y ? 0.5 : 1.0) * (rec.pij == rec.pkl ? 0.5 : 1.0);
-    const double* v = out + rec.out;
-    const int sj = ni, sk = ni * nj, sl = ni * nj * nk;
-    for (int j = 0; j < nj; ++j)
-      for (int i = 0; i < ni; ++i) {
-        double tj = 0.0;  // A[i,j]
-        for (int l = 0; l < nl; ++l)
-          for (int k = 0; k < nk; ++k) tj += v[i + j * sj + k * sk + l * sl] * dm[(size_t)(k0 + k) * nao + l0 + l];
-        if (A) atomicAdd(A + (size_t)(i0 + i) * nao + j0 + j, 2.0 * s * tj);
+// The same contraction with compile-time ket extents, each block element read once.  A group of G lanes
+// (the power of two from nij = ni*nj up, at most a warp) takes one quartet: lane <-> (i,j) (several of
+// them in turn where nij > 32), and walks the block's (k,l) elements, consecutive lanes reading
+// consecutive doubles.  Per element x it adds x D[k,l] to its A[i,j] sum, x D[j,l] and x D[i,l] to two
+// sums per k, x D[j,k] and x D[i,k] to two sums per l (all in registers), and the group reduces x D[i,j]
+// over its lanes into A[k,l] (halving_sum: about NK shuffles per l).  The per-(i,j) sums then meet in
+// shared memory, where they are reduced over j (i) before one atomic per element of B[i,kl] (B[j,kl]).
+// Consecutive quartets of a tile row share their (ij) pair, so a group takes runs of `run` records (up to
+// kJkRun, fewer where the records would not give every resident warp work) and adds A[i,j] once per run
+// and pair.
+//
+// Bound: the atomics, about (nk + nl)(ni + nj) + nk nl per quartet, at the L2's rate.  J+K of 120
+// s/p/d/f atoms (5.7e9 integrals): 139 ms of contraction with six passes over each block, 68 ms so.
+constexpr int kJkRun = 16;
+constexpr int kJkWarps = 4;
+
+// doubles of shared memory per group: D[k,l], A[k,l], A[i,j] and the per-(i,j) sums
+__host__ __device__ constexpr int jk_group_doubles(int nij, int nk, int nl) {
+  return 2 * nk * nl + nij + nij * 2 * (nk + nl);
+}
+
+// Sums p[0..N) over the group of G lanes starting at a multiple of G: where G >= 2, each step sends one
+// half of the values still held to the lane a power of two away and keeps the other half.  On return p[0]
+// is the group's sum of value `*which`; lanes with equal `*which` hold the same sum.
+template <int N>
+__device__ __forceinline__ void halving_sum(double (&p)[N], int G, unsigned mask, int lane, int* which) {
+  static_assert((N & (N - 1)) == 0, "padded to a power of two");
+  int w = 0, o = G >> 1;
+  if constexpr (N > 1) {
+    double h[N / 2];
+    if (o > 0) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int n = 0; n < N / 2; ++n) {
+        const double keep = up ? p[n + N / 2] : p[n], send = up ? p[n] : p[n + N / 2];
+        h[n] = keep + __shfl_xor_sync(mask, send, o);
       }
-    if (A)
-      for (int l = 0; l < nl; ++l)
-        for (int k = 0; k < nk; ++k) {
-          double t = 0.0;
-          for (int j = 0; j < nj; ++j)
-            for (int i = 0; i < ni; ++i) t += v[i + j * sj + k * sk + l * sl] * dm[(size_t)(i0 + i) * nao + j0 + j];
-          atomicAdd(A + (size_t)(k0 + k) * nao + l0 + l, 2.0 * s * t);
-        }
-    if (B) {
-      for (int k = 0; k < nk; ++k) {
-        for (int i = 0; i < ni; ++i) {  // B[i,k] += s sum_jl v D[j,l]
-          double t = 0.0;
-          for (int l = 0; l < nl; ++l)
-            for (int j = 0; j < nj; ++j) t += v[i + j * sj + k * sk + l * sl] * dm[(size_t)(j0 + j) * nao + l0 + l];
-          atomicAdd(B + (size_t)(i0 + i) * nao + k0 + k, s * t);
-        }
-        for (int j = 0; j < nj; ++j) {  // B[j,k] += s sum_il v D[i,l]
-          double t = 0.0;
-          for (int l = 0; l < nl; ++l)
-            for (int i = 0; i < ni; ++i) t += v[i + j * sj + k * sk + l * sl] * dm[(size_t)(i0 + i) * nao + l0 + l];
-          atomicAdd(B + (size_t)(j0 + j) * nao + k0 + k, s * t);
-        }
-      }
-      for (int l = 0; l < nl; ++l) {
-        for (int i = 0; i < ni; ++i) {  // B[i,l] += s sum_jk v D[j,k]
-          double t = 0.0;
-          for (int k = 0; k < nk; ++k)
-            for (int j = 0; j < nj; ++j) t += v[i + j * sj + k * sk + l * sl] * dm[(size_t)(j0 + j) * nao + k0 + k];
-          atomicAdd(B + (size_t)(i0 + i) * nao + l0 + l, s * t);
-        }
-        for (int j = 0; j < nj; ++j) {  // B[j,l] += s sum_ik v D[i,k]
-          double t = 0.0;
-          for (int k = 0; k < nk; ++k)
-            for (int i = 0; i < ni; ++i) t += v[i + j * sj + k * sk + l * sl] * dm[(size_t)(i0 + i) * nao + k0 + k];
-          atomicAdd(B + (size_t)(j0 + j) * nao + l0 + l, s * t);
-        }
-      }
+      w = up ? N / 2 : 0;
+      int sub = 0;
+      halving_sum<N / 2>(h, o, mask, lane, &sub);
+      p[0] = h[0];
+      *which = w + sub;
+      return;
     }
+    *which = 0;  // one lane left with several values: the caller reads p[0..N)
+  } else {
+    for (; o > 0; o >>= 1) p[0] += __shfl_xor_sync(mask, p[0], o);
+    *which = 0;
+  }
+}
+
+template <int NK, int NL>
+__global__ void __launch_bounds__(32 * kJkWarps)
+    jk_contract_group_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ psh,
+                             const int* __restrict__ aoloc, const double* __restrict__ out,
+                             const double* __restrict__ dm, int nao, double* __restrict__ A, double* __restrict__ B,
+                             int ni, int nj, int G, int run) {
+  constexpr int NP = NK <= 1 ? 1 : NK <= 2 ? 2 : NK <= 4 ? 4 : NK <= 8 ? 8 : 16;
+  constexpr int NKL = NK + NL;
+  extern __shared__ double sm[];
+  const int nij = ni * nj;
+  const int lane = threadIdx.x & 31, g = lane & (G - 1);
+  const unsigned mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
+  double* s_dkl = sm + (size_t)(threadIdx.x / G) * jk_group_doubles(nij, NK, NL);
+  double* s_akl = s_dkl + NK * NL;
+  double* s_aij = s_akl + NK * NL;
+  double* s_t = s_aij + nij;  // [2 * NKL][nij]: sums over l with D[j,l], over k with D[j,k]; with D[i,l], D[i,k]
+  const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
+  const long long ngroups = (long long)gridDim.x * blockDim.x / G;
+  for (long long base = gid * run; base < nrec; base += ngroups * run) {
+    const long long rend = base + run < nrec ? base + run : nrec;
+    int cur = -1;  // the (ij) pair whose A[i,j] sums s_aij holds
+    int i0 = 0, j0 = 0;
+    double sij = 0;
+    for (long long r = base; r < rend; ++r) {
+      const QuartetRec rec = recs[r];
+      const int2 cd = psh[rec.pkl];
+      const int k0 = aoloc[cd.x], l0 = aoloc[cd.y];
+      if (rec.pij != cur) {
+        if (cur >= 0 && A)
+          for (int e = g; e < nij; e += G) atomicAdd(A + (size_t)(i0 + e % ni) * nao + j0 + e / ni, s_aij[e]);
+        const int2 ab = psh[rec.pij];
+        i0 = aoloc[ab.x];
+        j0 = aoloc[ab.y];
+        sij = ab.x == ab.y ? 0.5 : 1.0;
+        cur = rec.pij;
+        for (int e = g; e < nij; e += G) s_aij[e] = 0.0;
+      }
+      const double s = sij * (cd.x == cd.y ? 0.5 : 1.0) * (rec.pij == rec.pkl ? 0.5 : 1.0);
+      for (int e = g; e < NK * NL; e += G) {
+        s_dkl[e] = dm[(size_t)(k0 + e % NK) * nao + l0 + e / NK];
+        s_akl[e] = 0.0;
+      }
+      __syncwarp(mask);
+      for (int ij0 = 0; ij0 < nij; ij0 += G) {
+        const int ij = ij0 + g;
+        const bool on = ij < nij;
+        const int i = on ? ij % ni : 0, j = on ? ij / ni : 0;
+        const double* v = out + rec.out + (on ? ij : 0);
+        const double* di = dm + (size_t)(i0 + i) * nao;
+        const double* dj = dm + (size_t)(j0 + j) * nao;
+        const double dij = di[j0 + j];
+        double djk[NK], dik[NK], t[NK], u[NK];
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+          djk[k] = dj[k0 + k];
+          dik[k] = di[k0 + k];
+          t[k] = u[k] = 0.0;
+        }
+        double aij = 0.0;
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+          const double djl = dj[l0 + l], dil = di[l0 + l];
+          double sl = 0.0, wl = 0.0, p[NP];
+#pragma unroll
+          for (int k = 0; k < NK; ++k) {
+            const double x = on ? v[(size_t)nij * (k + NK * l)] : 0.0;
+            aij = fma(x, s_dkl[k + NK * l], aij);
+            t[k] = fma(x, djl, t[k]);
+            u[k] = fma(x, dil, u[k]);
+            sl = fma(x, djk[k], sl);
+            wl = fma(x, dik[k], wl);
+            p[k] = x * dij;
+          }
+#pragma unroll
+          for (int k = NK; k < NP; ++k) p[k] = 0.0;
+          if (on) {
+            s_t[(NK + l) * nij + ij] = sl;
+            s_t[(NKL + NK + l) * nij + ij] = wl;
+          }
+          if (G >= NP) {  // one value per lane is left; the first lane of each value adds it up
+            int w;
+            halving_sum<NP>(p, G, mask, g, &w);
+            if (w < NK && (g & (G / NP - 1)) == 0) s_akl[w + NK * l] += p[0];
+          } else {
+#pragma unroll
+            for (int k = 0; k < NK; ++k) {
+              for (int o = G >> 1; o > 0; o >>= 1) p[k] += __shfl_xor_sync(mask, p[k], o);
+              if (g == 0) s_akl[k + NK * l] += p[k];
+            }
+          }
+        }
+        if (on) {
+          s_aij[ij] = fma(2.0 * s, aij, s_aij[ij]);
+#pragma unroll
+          for (int k = 0; k < NK; ++k) {
+            s_t[k * nij + ij] = t[k];
+            s_t[(NKL + k) * nij + ij] = u[k];
+          }
+        }
+      }
+      __syncwarp(mask);
+      if (A)
+        for (int e = g; e < NK * NL; e += G)
+          atomicAdd(A + (size_t)(k0 + e % NK) * nao + l0 + e / NK, 2.0 * s * s_akl[e]);
+      if (B) {
+        for (int e = g; e < ni * NKL; e += G) {  // B[i, k or l]: sums over j
+          const int i = e % ni, c = e / ni;
+          const double* x = s_t + c * nij + i;
+          double sum = 0.0;
+          for (int j = 0; j < nj; ++j) sum += x[ni * j];
+          atomicAdd(B + (size_t)(i0 + i) * nao + (c < NK ? k0 + c : l0 + c - NK), s * sum);
+        }
+        for (int e = g; e < nj * NKL; e += G) {  // B[j, k or l]: sums over i
+          const int j = e % nj, c = e / nj;
+          const double* x = s_t + (NKL + c) * nij + ni * j;
+          double sum = 0.0;
+          for (int i = 0; i < ni; ++i) sum += x[i];
+          atomicAdd(B + (size_t)(j0 + j) * nao + (c < NK ? k0 + c : l0 + c - NK), s * sum);
+        }
+      }
+      __syncwarp(mask);
+    }
+    if (cur >= 0 && A)
+      for (int e = g; e < nij; e += G) atomicAdd(A + (size_t)(i0 + e % ni) * nao + j0 + e / ni, s_aij[e]);
+    __syncwarp(mask);
   }
 }
 
@@ -344,16 +462,45 @@ cudaError_t launch_block_absmax_sqrt(const QuartetRec* recs, long long nrec, con
   return cudaGetLastError();
 }
 
+template <int NK, int NL>
+static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
+                                   const double* out, const double* dm, int nao, double* A, double* B,
+                                   cudaStream_t stream, int ni, int nj) {
+  int G = 1;
+  while (G < 32 && G < ni * nj) G *= 2;
+  const size_t smem = sizeof(double) * (size_t)jk_group_doubles(ni * nj, NK, NL) * (32 * kJkWarps / G);
+  auto kern = jk_contract_group_kernel<NK, NL>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const long long resident = 148LL * 16 * (32 / G);  // groups, 16 warps per SM
+  const int run = (int)std::max(1LL, std::min<long long>(kJkRun, nrec / (2 * resident)));
+  const long long per_block = 32LL * kJkWarps / G * run;
+  long long blocks = (nrec + per_block - 1) / per_block;
+  if (blocks > 148LL * 64) blocks = 148LL * 64;
+  kern<<<(unsigned)blocks, 32 * kJkWarps, smem, stream>>>(recs, nrec, psh, aoloc, out, dm, nao, A, B, ni, nj, G, run);
+  return cudaGetLastError();
+}
+
+// One class segment, blocks ni x nj x nk x nl.  Ket extents up to 10 have their own kernel (sph 1..9,
+// cart 1..10); cartesian g kets (15 functions: the sums of one lane no longer fit registers) keep the
+// general kernel.
 cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
                                const double* out, const double* dm, int nao, double* A, double* B, cudaStream_t stream,
-                               int block_elems) {
+                               int ni, int nj, int nk, int nl) {
   if (nrec <= 0) return cudaSuccess;
-  if (block_elems > 0 && block_elems <= 32) {
-    long long blocks = (nrec + 127) / 128;
-    if (blocks > 148LL * 64) blocks = 148LL * 64;
-    jk_contract_small_kernel<<<(unsigned)blocks, 128, 0, stream>>>(recs, nrec, psh, aoloc, out, dm, nao, A, B);
-    return cudaGetLastError();
+#define CINTX_JK(K, L) \
+  if (nk == K && nl == L) return launch_jk_group<K, L>(recs, nrec, psh, aoloc, out, dm, nao, A, B, stream, ni, nj);
+  if (jk_group_doubles(ni * nj, nk, nl) * sizeof(double) * kJkWarps <= 200 * 1024) {
+    CINTX_JK(1, 1) CINTX_JK(3, 1) CINTX_JK(3, 3)
+    CINTX_JK(5, 1) CINTX_JK(5, 3) CINTX_JK(5, 5)
+    CINTX_JK(6, 1) CINTX_JK(6, 3) CINTX_JK(6, 6)
+    CINTX_JK(7, 1) CINTX_JK(7, 3) CINTX_JK(7, 5) CINTX_JK(7, 7)
+    CINTX_JK(9, 1) CINTX_JK(9, 3) CINTX_JK(9, 5) CINTX_JK(9, 7) CINTX_JK(9, 9)
+    CINTX_JK(10, 1) CINTX_JK(10, 3) CINTX_JK(10, 6) CINTX_JK(10, 10)
   }
+#undef CINTX_JK
   long long blocks = (nrec * 32 + 255) / 256;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
   jk_contract_kernel<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, psh, aoloc, out, dm, nao, A, B);
