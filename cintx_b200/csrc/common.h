@@ -17,8 +17,9 @@ __host__ __device__ constexpr int cintx_rys_xmax(int n) {
 }
 
 // One primitive pair (a, b) of an oriented shell pair (i, j), after exponent screening.
-// kab folds exp(-a_i a_j/a_ij |A-B|^2), both contraction coefficients (single contraction)
-// and the pair's share of libcint's common factor sqrt(2 pi^2.5) * fac_sp(li) * fac_sp(lj).
+// kab folds exp(-a_i a_j/a_ij |A-B|^2), both contraction coefficients (single contraction), 1 / a_ij
+// and the pair's share of libcint's common factor sqrt(2 pi^2.5) * fac_sp(li) * fac_sp(lj), so that a
+// primitive quartet's prefactor is kab_ij kab_kl / sqrt(a_ij + a_kl).
 // When q is set, a shell pair's primitive pairs are sorted by decreasing q, so a primitive
 // quartet loop can stop at the first pair whose bound q_ab * q_cd falls below its threshold.
 struct __align__(64) PrimPair {
@@ -69,7 +70,7 @@ struct OutStrides {
 
 // Device Rys table (see gen_rys_table.py for the layout).
 struct RysTable {
-  const double* poly[CINTX_NRMAX + 1];  // [n] -> [xmax][DEG+1][2n]
+  const double* poly[CINTX_NRMAX + 1];  // [n] -> [xmax + 1][2n][DEG+1] (rys_roots.cuh)
   const double* asym[CINTX_NRMAX + 1];  // [n] -> h_r^2 (n), W_r (n)
   int xmax[CINTX_NRMAX + 1];
 };

@@ -64,7 +64,7 @@ struct Ip1Shape {
   static constexpr int GROUP_DOUBLES = (GROUP_DOUBLES_RAW + 1) & ~1;  // 16-byte groups
   // one-lane groups stage their root table in shared memory (as the plain kernel's one-lane classes)
   static constexpr bool STAGE_TABLE = S == 1 && NR <= 3;
-  static constexpr int TABLE_DOUBLES = STAGE_TABLE ? cintx_rys_xmax(NR) * rys_stage_stride(NR) : 0;
+  static constexpr int TABLE_DOUBLES = STAGE_TABLE ? rys_intervals(NR) * rys_stage_stride(NR) : 0;
   // groups per block: up to 128 threads, as many groups as 200 KB of shared memory holds
   static constexpr int QFIT = S == 1 ? 128 : (200 * 1024) / (GROUP_DOUBLES * 8);
   static constexpr int QWANT = S >= 128 ? 1 : 128 / S;
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
     constexpr int W = NR * RYS_NC, WP = rys_stage_stride(NR) / 2;  // double2 per interval, per stride
     const double2* src = reinterpret_cast<const double2*>(rys.poly[NR]);
     double2* dst = reinterpret_cast<double2*>(smem);
-    for (int i = threadIdx.x; i < cintx_rys_xmax(NR) * W; i += blockDim.x) dst[(i / W) * WP + i % W] = __ldg(src + i);
+    for (int i = threadIdx.x; i < rys_intervals(NR) * W; i += blockDim.x) dst[(i / W) * WP + i % W] = __ldg(src + i);
     __syncthreads();
   }
 
@@ -186,22 +186,20 @@ __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
         const PrimPair pi = prims[pij.prim_off + a];
         if (pi.cce + pk.cce > expcutoff) continue;  // CINT2e_loop eijcutoff (cint2e.c:700-712)
         const double aij = pi.aij, akl = pk.aij;
-        const double rs = rsqrt(aij + akl);
-        const double inv_aijkl = rs * rs;
-        const double inv_a1 = 4.0 * pi.half_inv * pk.half_inv;
         const double pqx = pi.px - pk.px, pqy = pi.py - pk.py, pqz = pi.pz - pk.pz;
-        const double x = aij * akl * inv_aijkl * (pqx * pqx + pqy * pqy + pqz * pqz);
-        const double fac = pi.kab * pk.kab * rs * inv_a1;
+        const RysPoint pt =
+            rys_point(aij * akl * (pqx * pqx + pqy * pqy + pqz * pqz), aij + akl, cintx_rys_xmax(NR));
+        const double fac = pi.kab * pk.kab * pt.r;
         const double pax = pi.px - pij.ax, pay = pi.py - pij.ay, paz = pi.pz - pij.az;
         const double ai2 = pi.q;  // 2 a_i of this primitive pair's i primitive
         if constexpr (S == 1) {
           double t2[NR], w[NR];
-          if constexpr (SH::STAGE_TABLE) rys_all_staged<NR>(smem, rys, x, t2, w);
-          else rys_all<NR>(rys, x, t2, w);
+          if constexpr (SH::STAGE_TABLE) rys_all_staged<NR>(smem, pt, t2, w);
+          else rys_all_at<NR>(rys, pt, t2, w);
 #pragma unroll
           for (int r = 0; r < NR; ++r) {
             double gg[3 * GSZ];
-            const double rt_aa = t2[r] * inv_aijkl;
+            const double rt_aa = t2[r] * pt.r2;
             const double b00 = 0.5 * rt_aa;
             const double b10 = pi.half_inv * (1.0 - rt_aa * akl);
             const double b01 = pk.half_inv * (1.0 - rt_aa * aij);
@@ -227,11 +225,11 @@ __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
             });
           }
         } else {
-          for (int f = lane; f < 2 * NR; f += S) s_roots[f] = rys_fn(rys, NR, f, x);
+          for (int f = lane; f < 2 * NR; f += S) s_roots[f] = rys_fn_at<NR>(rys, f, pt);
           group_sync<S>(group);
           for (int task = lane; task < 3 * NR; task += S) {
             const int axis = task / NR, r = task % NR;
-            const double rt_aa = s_roots[r] * inv_aijkl;
+            const double rt_aa = s_roots[r] * pt.r2;
             const double b00 = 0.5 * rt_aa;
             const double b10 = pi.half_inv * (1.0 - rt_aa * akl);
             const double b01 = pk.half_inv * (1.0 - rt_aa * aij);

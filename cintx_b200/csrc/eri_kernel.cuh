@@ -154,7 +154,7 @@ struct EriShape {
   // (multi-lane groups evaluate each root once per group; a per-block copy there costs more
   // occupancy than it saves, measured)
   static constexpr bool STAGE_TABLE = S == 1 && NR <= 3;
-  static constexpr int TABLE_DOUBLES = STAGE_TABLE ? cintx_rys_xmax(NR) * rys_stage_stride(NR) : 0;
+  static constexpr int TABLE_DOUBLES = STAGE_TABLE ? rys_intervals(NR) * rys_stage_stride(NR) : 0;
   static constexpr int SMEM_BYTES = Q * B_GROUP + TABLE_DOUBLES * 8;
   static constexpr bool IS_SLICE = SLICE;
   static constexpr int NPASS = PASSES;
@@ -502,30 +502,25 @@ __device__ __forceinline__ void prim_loop_one_lane(const ShellPair& pij, const S
       if (pi.q < qthr) break;
       if (pi.cce + pk.cce > expcutoff) continue;  // CINT2e_loop eijcutoff (cint2e.c:700-712)
       const double aij = pi.aij, akl = pk.aij;
-      const double aijkl = aij + akl;
-      const double rs = rsqrt(aijkl);
-      const double inv_aijkl = rs * rs;
-      const double a1 = aij * akl;
-      const double inv_a1 = 4.0 * pi.half_inv * pk.half_inv;
       const double pqx = pi.px - pk.px, pqy = pi.py - pk.py, pqz = pi.pz - pk.pz;
       const double rr = pqx * pqx + pqy * pqy + pqz * pqz;
-      const double x = a1 * inv_aijkl * rr;
-      const double fac = pi.kab * pk.kab * rs * inv_a1;
+      RysPoint pt;  // t2 and w below still want its factors r2 and r
       double t2[NR], w[NR];
       if (rb) {  // roots precomputed for this primitive quartet (learned-root plans)
+        pt.r = rsqrt(aij + akl);
+        pt.r2 = pt.r * pt.r;
         const double* r = rb + (size_t)(b * pij.nprim + a) * (2 * NR);
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
           t2[i] = r[i];
           w[i] = r[NR + i];
         }
-      } else if constexpr (SH::STAGE_TABLE) {
-        if constexpr (SSSS) rys_all_staged<NR, NR, 2 * NR>(tab, rys, x, t2, w);
-        else rys_all_staged<NR>(tab, rys, x, t2, w);
       } else {
-        if constexpr (SSSS) rys_all<NR, NR, 2 * NR>(rys, x, t2, w);
-        else rys_all<NR>(rys, x, t2, w);
+        pt = rys_point(aij * akl * rr, aij + akl, cintx_rys_xmax(NR));
+        if constexpr (SH::STAGE_TABLE) rys_all_staged<NR, SSSS ? NR : 0>(tab, pt, t2, w);
+        else rys_all_at<NR, SSSS ? NR : 0>(rys, pt, t2, w);
       }
+      const double fac = pi.kab * pk.kab * pt.r;
       if constexpr (SSSS) {
         acc[0][0] = fma(w[0], fac, acc[0][0]);  // (ss|ss) needs the weight only
       } else {
@@ -541,7 +536,7 @@ __device__ __forceinline__ void prim_loop_one_lane(const ShellPair& pij, const S
         }
         auto root_body = [&](const int r) {
           R gg[3 * GSZ];
-          const double rt_aa = t2[r] * inv_aijkl;
+          const double rt_aa = t2[r] * pt.r2;
           const double b00 = 0.5 * rt_aa;
           const double b10 = pi.half_inv * (1.0 - rt_aa * akl);
           const double b01 = pk.half_inv * (1.0 - rt_aa * aij);
@@ -631,7 +626,7 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
     constexpr int W = NR * RYS_NC, WP = rys_stage_stride(NR) / 2;  // double2 per block, per stride
     const double2* src = reinterpret_cast<const double2*>(rys.poly[NR]);
     double2* dst = reinterpret_cast<double2*>(smem);
-    for (int i = threadIdx.x; i < cintx_rys_xmax(NR) * W; i += blockDim.x) dst[(i / W) * WP + i % W] = __ldg(src + i);
+    for (int i = threadIdx.x; i < rys_intervals(NR) * W; i += blockDim.x) dst[(i / W) * WP + i % W] = __ldg(src + i);
     __syncthreads();
   }
 
@@ -721,33 +716,30 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
         if (pi.q < qthr) break;
         if (pi.cce + pk.cce > expcutoff) continue;  // CINT2e_loop eijcutoff (cint2e.c:700-712)
         const double aij = pi.aij, akl = pk.aij;
-        const double aijkl = aij + akl;
-        const double rs = rsqrt(aijkl);
-        const double inv_aijkl = rs * rs;
-        const double a1 = aij * akl;
-        const double inv_a1 = 4.0 * pi.half_inv * pk.half_inv;
         const double pqx = pi.px - pk.px, pqy = pi.py - pk.py, pqz = pi.pz - pk.pz;
         const double rr = pqx * pqx + pqy * pqy + pqz * pqz;
-        const double x = a1 * inv_aijkl * rr;
-        const double fac = pi.kab * pk.kab * rs * inv_a1;
         const double pax = pi.px - pij.ax, pay = pi.py - pij.ay, paz = pi.pz - pij.az;
 
-        // roots: the group's lanes split the 2*NR table polynomials (or copy precomputed ones)
+        // roots: the group's lanes split the 2*NR table polynomials (or copy precomputed ones); the
+        // values in s_roots still want the factors r2 and r of the point
+        RysPoint pt;
         if (rb) {
+          pt.r = rsqrt(aij + akl);
+          pt.r2 = pt.r * pt.r;
           const double* r = rb + (size_t)(b * pij.nprim + a) * (2 * NR);
           for (int f = lane; f < 2 * NR; f += S) s_roots[f] = r[f];
-        } else if constexpr (SH::STAGE_TABLE) {
-          for (int f = lane; f < 2 * NR; f += S) s_roots[f] = rys_fn_staged<NR>(smem, rys, f, x);
         } else {
-          for (int f = lane; f < 2 * NR; f += S) s_roots[f] = rys_fn(rys, NR, f, x);
+          pt = rys_point(aij * akl * rr, aij + akl, cintx_rys_xmax(NR));
+          for (int f = lane; f < 2 * NR; f += S)
+            s_roots[f] = SH::STAGE_TABLE ? rys_fn_staged<NR>(smem, f, pt) : rys_fn_at<NR>(rys, f, pt);
         }
+        const double fac = pi.kab * pk.kab * pt.r;
         group_sync<S>(group);
         // (axis, root) recurrences, one per lane; coefficients in FP64, recurrences in R
         for (int tp = lane; tp < 3 * NR * SH::NPARTS; tp += S) {
           const int task = tp / SH::NPARTS, part = tp % SH::NPARTS;
           const int axis = task / NR, r = task % NR;
-          const double t2 = s_roots[r];
-          const double rt_aa = t2 * inv_aijkl;
+          const double rt_aa = s_roots[r] * pt.r2;
           const double b00 = 0.5 * rt_aa;
           const double b10 = pi.half_inv * (1.0 - rt_aa * akl);
           const double b01 = pk.half_inv * (1.0 - rt_aa * aij);

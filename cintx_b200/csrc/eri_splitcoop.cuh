@@ -180,23 +180,23 @@ __global__ void __launch_bounds__(splitcoop_dims(LI, LJ, LK, LL, ACC).BLOCK, spl
         if (pi.q < qthr) break;
         if (pi.cce + pk.cce > expcutoff) continue;  // CINT2e_loop eijcutoff (cint2e.c:700-712)
         const double aij = pi.aij, akl = pk.aij;
-        const double rs = rsqrt(aij + akl);
-        const double inv_aijkl = rs * rs;
-        const double inv_a1 = 4.0 * pi.half_inv * pk.half_inv;
         const double pqx = pi.px - pk.px, pqy = pi.py - pk.py, pqz = pi.pz - pk.pz;
-        const double x = aij * akl * inv_aijkl * (pqx * pqx + pqy * pqy + pqz * pqz);
-        const double fac = pi.kab * pk.kab * rs * inv_a1;
+        RysPoint pt;
         if (rb) {
+          pt.r = rsqrt(aij + akl);
+          pt.r2 = pt.r * pt.r;
           const double* r = rb + (size_t)(b * pij.nprim + a) * (2 * NR);
           for (int f = lane; f < 2 * NR; f += S) s_roots[f] = r[f];
         } else {
-          for (int f = lane; f < 2 * NR; f += S) s_roots[f] = rys_fn(rys, NR, f, x);
+          pt = rys_point(aij * akl * (pqx * pqx + pqy * pqy + pqz * pqz), aij + akl, cintx_rys_xmax(NR));
+          for (int f = lane; f < 2 * NR; f += S) s_roots[f] = rys_fn_at<NR>(rys, f, pt);
         }
+        const double fac = pi.kab * pk.kab * pt.r;
         group_sync<S>(group);
         // V: the 2D tables
         for (int task = lane; task < 3 * NR; task += S) {
           const int axis = task / NR, r = task % NR;
-          const double rt_aa = s_roots[r] * inv_aijkl;
+          const double rt_aa = s_roots[r] * pt.r2;
           const double b00 = 0.5 * rt_aa;
           const double b10 = pi.half_inv * (1.0 - rt_aa * akl);
           const double b01 = pk.half_inv * (1.0 - rt_aa * aij);

@@ -192,9 +192,9 @@ void build_pair(const Basis& B, int a, int b, double expcutoff, PairHost& out, i
       pp.px = A.r[0];
       pp.py = A.r[1];
       pp.pz = A.r[2];
-      pp.kab = A.coef[(size_t)ca * A.nprim + p] * sq_common * common_fac_sp(A.l);
-      pp.cce = 0;
       pp.half_inv = 0.5 / A.exps[p];
+      pp.kab = A.coef[(size_t)ca * A.nprim + p] * sq_common * common_fac_sp(A.l) * (2.0 * pp.half_inv);
+      pp.cce = 0;
       out.prims.push_back(pp);
       out.pa.push_back(p);
       out.pb.push_back(0);
@@ -228,7 +228,7 @@ void build_pair(const Basis& B, int a, int b, double expcutoff, PairHost& out, i
         pp.px = A.r[0] - wj * d[0];
         pp.py = A.r[1] - wj * d[1];
         pp.pz = A.r[2] - wj * d[2];
-        pp.kab = exp(-eij) * cprod * fac;
+        pp.kab = exp(-eij) * cprod * fac * inv;
         pp.cce = cce;
         pp.half_inv = 0.5 * inv;
         out.prims.push_back(pp);

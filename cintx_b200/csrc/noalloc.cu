@@ -29,7 +29,7 @@
 
 namespace {
 
-constexpr size_t kRysTableDoubles = 87040;  // >= doubles in the device layout of the Rys table
+constexpr size_t kRysTableDoubles = 88320;  // >= doubles in the device layout of the Rys table
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[CINTX_NOALLOC_SCRATCH_BYTES];
 static __device__ __align__(256) double g_noalloc_rys[kRysTableDoubles];

@@ -1,8 +1,10 @@
 // Device copy of the Rys root table (rys_table.bin, embedded at link time) and its upload.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 #include "common.h"
 #include "host_internal.h"
@@ -23,9 +25,11 @@ namespace cintx {
 
 // Reads the embedded table: checks its header against the layout the kernels are compiled for
 // (order >= CINTX_NRMAX, degree CINTX_RYS_DEG, the interval counts of cintx_rys_xmax, a payload
-// of exactly the size the header implies), and returns the payload transposed from the file's
-// [degree][function] order to the [function][degree] order the device reads, with each order's
-// polynomial block and asymptotic constants as offsets (doubles) into it.  0 on success.
+// of exactly the size the header implies), and returns it in the device layout of rys_roots.cuh: each
+// order's intervals transposed from the file's [degree][function] order to [function][degree], the
+// coefficients rescaled from z = 2d to d (powers of two: exact), and one interval more, past the
+// table's end, whose functions are the constants of the large-x form; then the asymptotic constants.
+// offs: each order's block and constants (doubles into the payload).  0 on success.
 int rys_table_image(std::vector<double>& payload, RysTableOffsets& offs) {
   const unsigned char* p = cintx_rys_table_bin;
   const size_t nbytes = (size_t)(cintx_rys_table_bin_end - cintx_rys_table_bin);
@@ -42,29 +46,32 @@ int rys_table_image(std::vector<double>& payload, RysTableOffsets& offs) {
     total += (size_t)xmax * (deg + 1) * 2 * n + 2 * n;
   }
   if (sizeof(hdr) + total * sizeof(double) != nbytes) return 4;
-  payload.resize(total);
-  memcpy(payload.data(), p + sizeof(hdr), total * sizeof(double));
+  std::vector<double> file(total);
+  memcpy(file.data(), p + sizeof(hdr), total * sizeof(double));
   memset(&offs, 0, sizeof(offs));
-  size_t o = 0;
-  std::vector<double> tmp;
+  payload.clear();
   const int nc = deg + 1;
+  size_t asym = total;  // the constants follow the polynomials: 2n of each order
+  for (int n = 1; n <= nmax; ++n) asym -= 2 * n;
+  size_t o = 0, oa = asym;
   for (int n = 1; n <= nmax; ++n) {
     const int nf = 2 * n, xmax = (int)hdr[1 + n];
-    if (n <= CINTX_NRMAX) {
-      offs.poly[n] = o;
-      offs.xmax[n] = xmax;
-    }
-    for (int i = 0; i < xmax; ++i, o += (size_t)nf * nc) {
-      tmp.assign(payload.begin() + o, payload.begin() + o + (size_t)nf * nc);
-      for (int k = 0; k < nc; ++k)
-        for (int f = 0; f < nf; ++f) payload[o + (size_t)f * nc + k] = tmp[(size_t)k * nf + f];
-    }
+    if (n > CINTX_NRMAX) break;
+    offs.poly[n] = payload.size();
+    offs.xmax[n] = xmax;
+    for (int i = 0; i < xmax; ++i, o += (size_t)nf * nc)
+      for (int f = 0; f < nf; ++f)
+        for (int k = 0; k < nc; ++k) payload.push_back(ldexp(file[o + (size_t)k * nf + f], k));
+    for (int f = 0; f < nf; ++f, ++oa)
+      for (int k = 0; k < nc; ++k) payload.push_back(k == 0 ? file[oa] : 0.0);
   }
-  for (int n = 1; n <= nmax; ++n) {
-    if (n <= CINTX_NRMAX) offs.asym[n] = o;
-    o += 2 * n;
+  oa = asym;
+  for (int n = 1; n <= std::min(nmax, (int)CINTX_NRMAX); ++n) {
+    offs.asym[n] = payload.size();
+    payload.insert(payload.end(), file.begin() + oa, file.begin() + oa + 2 * n);
+    oa += 2 * n;
   }
-  return o == total ? 0 : 4;
+  return 0;
 }
 
 // Copies the table to the current device and fills *tab with its device pointers.
