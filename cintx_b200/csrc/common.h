@@ -40,12 +40,16 @@ struct __align__(16) ShellPair {
   int ish, jsh;          // shell ids
 };
 
-// One shell quartet of a launch: pairs (ij) and (kl) and the start of its output block.
+// One shell quartet of a launch: pairs (ij) and (kl), the start of its output block (doubles) in the low
+// 56 bits of `out`, and in the high 8 which of the launch's stride sets its block is laid out with (0 in
+// every list but explicit ones, whose tuples may name the shells of a class in any order).
 struct __align__(16) QuartetRec {
   int pij;
   int pkl;
-  long long out;  // offset in doubles
+  long long out;
 };
+__host__ __device__ inline long long rec_offset(const QuartetRec& r) { return r.out & ((1LL << 56) - 1); }
+__host__ __device__ inline int rec_strides(const QuartetRec& r) { return (int)((unsigned long long)r.out >> 56); }
 
 // A contiguous run [t0, t1) of one screened tile's row-major quartet numbering, generating
 // records rec_off.. of a merged class segment whose blocks start at out_off (doubles).
@@ -67,6 +71,37 @@ struct __align__(16) GenRange {
 struct OutStrides {
   long long s0, s1, s2, s3;
 };
+
+// The layouts of one launch's blocks, by rec_strides.
+struct StrideSet {
+  OutStrides s[8];
+};
+inline StrideSet one_stride(const OutStrides& st) {
+  StrideSet r{};
+  r.s[0] = st;
+  return r;
+}
+
+// The eight index orders a tuple list can name a class's shells in: bit 0, the kernel's first pair is
+// requested (second shell, first shell); bit 1, its second pair; bit 2, the kernel's second pair is
+// requested first.  `extent` are the functions (contractions included) along the kernel's axes; the
+// requested axes are laid out first fastest.
+inline int order_code(const int (&src)[4]) {
+  return (src[0] & 1) | ((src[2] & 1) << 1) | (src[0] >= 2 ? 4 : 0);
+}
+inline StrideSet order_strides(const long long (&extent)[4]) {
+  StrideSet r{};
+  for (int code = 0; code < 8; ++code) {
+    long long st[4], n = 1;
+    for (int x = 0; x < 4; ++x) {  // requested axis x: kernel pair and shell of it
+      const int pair = (x >> 1) ^ (code >> 2), second = (x & 1) ^ ((code >> pair) & 1);
+      st[2 * pair + second] = n;
+      n *= extent[2 * pair + second];
+    }
+    r.s[code] = OutStrides{st[0], st[1], st[2], st[3]};
+  }
+  return r;
+}
 
 // Device Rys table (see gen_rys_table.py for the layout).
 struct RysTable {

@@ -7,7 +7,7 @@
 namespace cintx {
 
 cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const QuartetRec* recs, int nrec,
-                         const ShellPair* pairs, const PrimPair* prims, double* out, OutStrides st,
+                         const ShellPair* pairs, const PrimPair* prims, double* out, const StrideSet& st,
                          double expcutoff, const RysTable& rys, cudaStream_t stream, bool fp32,
                          double prim_eps, int variant, const double* rootbuf, const long long* rootbase, int nsplit) {
   LaunchArgs a;

@@ -127,8 +127,8 @@ __device__ __forceinline__ void ip1_products(double (&acc)[3][NFI], const double
 template <int LI, int LJ, int LK, int LL, bool SPH>
 __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
     eri_ip1_kernel(const QuartetRec* __restrict__ recs, int nrec, const ShellPair* __restrict__ pairs,
-                   const PrimPair* __restrict__ prims, double* __restrict__ out, OutStrides st, long long scomp,
-                   double expcutoff, const __grid_constant__ RysTable rys, int nsplit) {
+                   const PrimPair* __restrict__ prims, double* __restrict__ out,
+                   const __grid_constant__ StrideSet sts, long long scomp, double expcutoff, const __grid_constant__ RysTable rys, int nsplit) {
   using SH = Ip1Shape<LI, LJ, LK, LL, SPH>;
   static_assert(ip1_shape_violation<SH>() == 0, "an index of this ip1 launch shape can leave its buffer");
   constexpr int S = SH::S, NR = SH::NR, GSZ = SH::GSZ, NFI = SH::NFI, TPT = SH::TPT;
@@ -278,6 +278,8 @@ __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
       }
     }
     // ---- transform each component to spherical and store ----
+    double* const obase = out + rec_offset(rec);
+    const OutStrides st = sts.s[rec_strides(rec)];
     if constexpr (S == 1) {
       const unsigned tmask = ns == 32 ? 0xffffffffu : (((1u << ns) - 1u) << (threadIdx.x & 31u & ~(unsigned)(ns - 1)));
       for (int o = ns >> 1; o > 0; o >>= 1) {
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
                 if (ci * cj * ck * cl != 0.0) v += ci * cj * ck * cl * acc[t][c][fi];
               }
             }
-            out[rec.out + c * scomp + mi * st.s0 + mj * st.s1 + mk * st.s2 + ml * st.s3] = v;
+            obase[c * scomp + mi * st.s0 + mj * st.s1 + mk * st.s2 + ml * st.s3] = v;
           });
       }
     } else {
@@ -317,7 +319,7 @@ __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
       team_sync(tn, team);  // every group's last products are read
 #pragma unroll 1
       for (int comp = 0; comp < 3; ++comp) {
-        double* const obase = out + rec.out + comp * scomp;
+        double* const cbase = obase + comp * scomp;
         auto stage_i = [&](auto cc) {  // this group's partial block, its i axis transformed
           constexpr int c = decltype(cc)::value;
 #pragma unroll
@@ -396,7 +398,7 @@ __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
             } else {
               v = cur[mijk + MIJK * ml];
             }
-            obase[mi * st.s0 + mj * st.s1 + mk * st.s2 + ml * st.s3] = v;
+            cbase[mi * st.s0 + mj * st.s1 + mk * st.s2 + ml * st.s3] = v;
           }
         }
         team_sync(tn, team);
@@ -411,7 +413,7 @@ struct Ip1Args {
   const ShellPair* pairs;
   const PrimPair* prims;
   double* out;
-  OutStrides st;
+  StrideSet st;
   long long scomp;
   double expcutoff;
   RysTable rys;

@@ -588,8 +588,8 @@ template <int LI, int LJ, int LK, int LL, bool SPH, class R = double, int ACC = 
 __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>::BLOCK,
                                   EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>::MINB)
     eri4c_kernel(const QuartetRec* __restrict__ recs, int nrec, const ShellPair* __restrict__ pairs,
-                 const PrimPair* __restrict__ prims, double* __restrict__ out, OutStrides st,
-                 double expcutoff, const __grid_constant__ RysTable rys, double* __restrict__ gscratch,
+                 const PrimPair* __restrict__ prims, double* __restrict__ out,
+                 const __grid_constant__ StrideSet sts, double expcutoff, const __grid_constant__ RysTable rys, double* __restrict__ gscratch,
                  double prim_eps, const double* __restrict__ rootbuf, const long long* __restrict__ rootbase,
                  int nsplit) {
   using SH = EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>;
@@ -805,7 +805,8 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
     }
 
     // ---- transform to spherical and store ----
-    double* const obase = out + rec.out;
+    double* const obase = out + rec_offset(rec);
+    const OutStrides st = sts.s[rec_strides(rec)];
     if constexpr (S == 1) {
       // whole block in registers: TPT == NTUP
 #pragma unroll

@@ -12,7 +12,7 @@ struct LaunchArgs {
   const ShellPair* pairs;
   const PrimPair* prims;
   double* out;
-  OutStrides st;
+  StrideSet st;
   double expcutoff;
   RysTable rys;
   cudaStream_t stream;

@@ -137,8 +137,8 @@ __device__ __forceinline__ void hrr_jl(double* __restrict__ dst, const double* _
 template <int LI, int LJ, int LK, int LL, int ACC>
 __global__ void __launch_bounds__(splitcoop_dims(LI, LJ, LK, LL, ACC).BLOCK, splitcoop_dims(LI, LJ, LK, LL, ACC).MINB)
     eri_splitcoop_kernel(const QuartetRec* __restrict__ recs, int nrec, const ShellPair* __restrict__ pairs,
-                         const PrimPair* __restrict__ prims, double* __restrict__ out, OutStrides st,
-                         double expcutoff, const __grid_constant__ RysTable rys, double prim_eps,
+                         const PrimPair* __restrict__ prims, double* __restrict__ out,
+                         const __grid_constant__ StrideSet sts, double expcutoff, const __grid_constant__ RysTable rys, double prim_eps,
                          const double* __restrict__ rootbuf, const long long* __restrict__ rootbase) {
   using SH = EriShape<LI, LJ, LK, LL, true, double, ACC, kSplitCoopRegs>;
   constexpr SplitCoopDims D = splitcoop_dims(LI, LJ, LK, LL, ACC);
@@ -239,7 +239,8 @@ __global__ void __launch_bounds__(splitcoop_dims(LI, LJ, LK, LL, ACC).BLOCK, spl
       }
     }
     // ---- transform to spherical and store (the default cooperative shape's stages) ----
-    double* const obase = out + rec.out;
+    double* const obase = out + rec_offset(rec);
+    const OutStrides st = sts.s[rec_strides(rec)];
     double* bufA = sg;
     double* bufB = bufA + SH::SM_BUFA;
 #pragma unroll

@@ -738,7 +738,7 @@ static int eval_call(int family, bool sph, double* out, int* dims, int* shls, in
   for (int c = 0; c < 4; ++c) *sv[c] = axstride[ori.src[c]];
   cudaError_t e = launch_class(ori.li, ori.lj, ori.lk, ori.ll, sph, (const QuartetRec*)(d + off_recs), (int)recs.size(),
                                (const ShellPair*)(d + off_pairs), (const PrimPair*)(d + off_prims),
-                               (double*)(d + off_out), st, cutoff, ds->rys, ts->stream, false, 0.0, 0, nullptr, nullptr,
+                               (double*)(d + off_out), one_stride(st), cutoff, ds->rys, ts->stream, false, 0.0, 0, nullptr, nullptr,
                                prim_split(ori.li, ori.lj, ori.lk, ori.ll, pwork, (long long)recs.size(), pmax).ns);
   if (e != cudaSuccess) {
     set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("kernel launch failed: ") + cudaGetErrorString(e));

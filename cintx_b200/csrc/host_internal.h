@@ -163,7 +163,7 @@ double flops_c2s(int li, int lj, int lk, int ll, bool sph);
 
 bool class_needs_scratch(int li, int lj, int lk, int ll, bool sph, int variant = 0);
 cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const QuartetRec* recs, int nrec,
-                         const ShellPair* pairs, const PrimPair* prims, double* out, OutStrides st,
+                         const ShellPair* pairs, const PrimPair* prims, double* out, const StrideSet& st,
                          double expcutoff, const RysTable& rys, cudaStream_t stream, bool fp32 = false,
                          double prim_eps = 0.0, int variant = 0, const double* rootbuf = nullptr,
                          const long long* rootbase = nullptr, int nsplit = 1);

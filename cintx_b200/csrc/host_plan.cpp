@@ -93,7 +93,8 @@ int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 
 struct Segment {
   int li, lj, lk, ll;
-  OutStrides st;
+  OutStrides st{};       // screened plans: every block's layout
+  int strides = -1;      // explicit plans: the plan's stride set of the records' layouts
   double expcutoff;
   // explicit: records at d_recs[rec0, rec0+nrec); screened: tile index and quartet range
   long long rec0 = 0;
@@ -164,6 +165,7 @@ struct CintxPlan {
   QuartetRec* d_recs = nullptr;    // explicit: all records; screened: one chunk's records
   long long rec_capacity = 0;
   char* d_tile_pool = nullptr;     // screened: every tile's rows, cols, prefix and colstart arrays
+  std::vector<StrideSet> stride_sets;  // explicit: one per segment class
   std::vector<QuartetRec> h_recs;  // explicit plans keep a host copy for chunk_quartets
   std::vector<int> h_tuples;       // explicit: requested tuples (4 per record, -1 for unit)
   CintxPlanStats stats{};
@@ -285,6 +287,7 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
     std::vector<int> tuples;
     double flops = 0;
     double work = 0, pmax = 0;  // primitive quartets: all, and of the largest record
+    long long extent[4];        // functions (contractions included) along the kernel's axes
   };
   PhaseLog plog("explicit plan");
   // 1. requested shells and block sizes (serial; the first bad shell index ends the plan)
@@ -426,10 +429,11 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
               r.pkl = swap ? id1 : id2;
               long long o2 = off;
               for (int x = 0; x < 4; ++x) o2 += (long long)cs[x] * ne[x] * ast[x];
-              r.out = o2;
+              r.out = o2 | ((long long)order_code(src) << 56);
               if (!last || last_key < k || k < last_key) {
                 last = &P.groups[k];
                 last_key = k;
+                for (int x = 0; x < 4; ++x) last->extent[x] = (long long)nc[src[x]] * ne[src[x]];
               }
               last->recs.push_back(r);
               for (int x = 0; x < 4; ++x) last->tuples.push_back(rs[x]);
@@ -493,34 +497,44 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
   long long rec0 = 0;
   std::vector<std::pair<const Group*, long long>> copies;  // (part group, first record)
   std::vector<std::pair<size_t, double>> heavy;            // segments split in two: (index, pmin)
+  // groups of one class and extents (they differ in the tuples' index order) are one segment: each
+  // record says which of the class's eight layouts its block has (order_strides)
+  std::vector<std::pair<double, double>> seg_work;  // primitive quartets: all, and of the largest record
+  const long long* seg_extent = nullptr;
   for (auto& kv : joined) {
-    Segment sg;
-    sg.li = kv.first.li;
-    sg.lj = kv.first.lj;
-    sg.lk = kv.first.lk;
-    sg.ll = kv.first.ll;
-    sg.st.s0 = kv.first.s0;
-    sg.st.s1 = kv.first.s1;
-    sg.st.s2 = kv.first.s2;
-    sg.st.s3 = kv.first.s3;
-    sg.expcutoff = cutoff;
-    sg.rec0 = rec0;
-    sg.nrec = 0;
-    sg.out_off = 0;
-    sg.flops = 0;
-    double work = 0, pmax = 0;
+    const GKey& k = kv.first;
+    const long long* extent = kv.second[0]->extent;
+    const Segment* prev = ch.segs.empty() ? nullptr : &ch.segs.back();
+    if (!prev || prev->li != k.li || prev->lj != k.lj || prev->lk != k.lk || prev->ll != k.ll ||
+        !std::equal(extent, extent + 4, seg_extent)) {
+      Segment sg;
+      sg.li = k.li;
+      sg.lj = k.lj;
+      sg.lk = k.lk;
+      sg.ll = k.ll;
+      sg.strides = (int)p->stride_sets.size();
+      p->stride_sets.push_back(order_strides({extent[0], extent[1], extent[2], extent[3]}));
+      sg.expcutoff = cutoff;
+      sg.rec0 = rec0;
+      ch.segs.push_back(sg);
+      seg_work.emplace_back(0.0, 0.0);
+      seg_extent = extent;
+    }
+    Segment& sg = ch.segs.back();
     for (const Group* g : kv.second) {
-      copies.emplace_back(g, rec0 + sg.nrec);
+      copies.emplace_back(g, rec0);
+      rec0 += (long long)g->recs.size();
       sg.nrec += (long long)g->recs.size();
       sg.flops += g->flops;
-      work += g->work;
-      pmax = std::max(pmax, g->pmax);
+      seg_work.back().first += g->work;
+      seg_work.back().second = std::max(seg_work.back().second, g->pmax);
     }
-    const PrimSplit ps = prim_split(sg.li, sg.lj, sg.lk, sg.ll, work, sg.nrec, pmax);
+  }
+  for (size_t i = 0; i < ch.segs.size(); ++i) {
+    Segment& sg = ch.segs[i];
+    const PrimSplit ps = prim_split(sg.li, sg.lj, sg.lk, sg.ll, seg_work[i].first, sg.nrec, seg_work[i].second);
     sg.nsplit = ps.ns;
-    if (ps.ns > 1 && ps.pmin > 0) heavy.emplace_back(ch.segs.size(), ps.pmin);
-    ch.segs.push_back(sg);
-    rec0 += sg.nrec;
+    if (ps.ns > 1 && ps.pmin > 0) heavy.emplace_back(i, ps.pmin);
   }
   {
     // the records and tuples of every part group into place, on host threads
@@ -620,7 +634,7 @@ static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStr
     const int nr = (int)std::min<long long>(nrec - r0, 1LL << 30);
     const bool rb = p->d_rootbuf && sg.tile == -1;  // learned roots: explicit plans only
     cudaError_t e = launch_class(sg.li, sg.lj, sg.lk, sg.ll, p->sph, recs + r0, nr, o->d_pairs, o->d_prims,
-                                 out_dev + sg.out_off, sg.st, sg.expcutoff, ds->rys, stream, sg.fp32, sg.prim_eps,
+                                 out_dev + sg.out_off, sg.strides >= 0 ? p->stride_sets[sg.strides] : one_stride(sg.st), sg.expcutoff, ds->rys, stream, sg.fp32, sg.prim_eps,
                                  sg.variant, rb ? p->d_rootbuf : nullptr, rb ? p->d_rootbase + sg.rec0 + r0 : nullptr,
                                  sg.nsplit);
     if (e != cudaSuccess) {
@@ -1640,7 +1654,7 @@ int compute_prim_schwarz(Opt* o) {
         st.s3 = st.s2 * ncart(la);
         for (long long q0 = 0; q0 < nrec && ok; q0 += 1LL << 30) {
           const int nr = (int)std::min<long long>(nrec - q0, 1LL << 30);
-          ok = launch_class(la, lb, la, lb, false, d_recs + r0 + q0, nr, d_tp, o->d_prims, d_out, st, 1e6, ds->rys,
+          ok = launch_class(la, lb, la, lb, false, d_recs + r0 + q0, nr, d_tp, o->d_prims, d_out, one_stride(st), 1e6, ds->rys,
                             ts->stream) == cudaSuccess;
           ts->launches++;
         }
@@ -1791,7 +1805,7 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
           for (int part = 0; part < 2 && ok; ++part) {
             const long long q0 = part ? rs : r0, q1 = part ? seg_end[g] : rs;
             if (q1 <= q0) continue;
-            ok = launch_class(la, lb, la, lb, true, d_recs + q0, (int)(q1 - q0), o->d_pairs, o->d_prims, d_out, st,
+            ok = launch_class(la, lb, la, lb, true, d_recs + q0, (int)(q1 - q0), o->d_pairs, o->d_prims, d_out, one_stride(st),
                               ecut, ds->rys, ts->stream, false, 0.0, 0, nullptr, nullptr, part ? 1 : ps.ns) ==
                  cudaSuccess;
             ts->launches++;

@@ -58,12 +58,12 @@ namespace {
 struct Ip1Work {
   std::vector<ShellPair> pairs;
   std::vector<PrimPair> prims;
-  struct Key {  // kernel class, output strides and component stride (the tuple's block size)
+  struct Key {  // kernel class and the extents of its axes (functions times contractions)
     int li, lj, lk, ll;
-    long long s0, s1, s2, s3, blk;
+    long long e[4];
     bool operator<(const Key& o) const {
-      return std::tie(li, lj, lk, ll, s0, s1, s2, s3, blk) <
-             std::tie(o.li, o.lj, o.lk, o.ll, o.s0, o.s1, o.s2, o.s3, o.blk);
+      return std::tie(li, lj, lk, ll, e[0], e[1], e[2], e[3]) <
+             std::tie(o.li, o.lj, o.lk, o.ll, o.e[0], o.e[1], o.e[2], o.e[3]);
     }
   };
   struct Group {
@@ -170,7 +170,10 @@ int ip1_build(const Basis& B, int nsh, const int* shls, int64_t n, bool sph, boo
             if (W.pair_min_cce[r.pij] + W.pair_min_cce[r.pkl] <= cutoff) W.any = true;
             r.out = off;
             for (int a = 0; a < 4; ++a) r.out += (long long)cs[a] * ne[a] * ast[a];
-            Ip1Work::Key k{l[0], l[1], l[src[2]], l[src[3]], ast[0], ast[1], ast[src[2]], ast[src[3]], st};
+            r.out |= (long long)order_code(src) << 56;
+            Ip1Work::Key k{l[0], l[1], l[src[2]], l[src[3]],
+                           {(long long)nc[0] * ne[0], (long long)nc[1] * ne[1], (long long)nc[src[2]] * ne[src[2]],
+                            (long long)nc[src[3]] * ne[src[3]]}};
             if (!last || last_key < k || k < last_key) {
               last = &W.groups[k];
               last_key = k;
@@ -265,11 +268,8 @@ int ip1_launch(const Ip1Work& W, bool sph, int nsh, const Basis& B, char* dev, c
       a.pairs = (const ShellPair*)dev;
       a.prims = (const PrimPair*)(dev + o_prims);
       a.out = out_dev;
-      a.st.s0 = k.s0;
-      a.st.s1 = k.s1;
-      a.st.s2 = k.s2;
-      a.st.s3 = k.s3;
-      a.scomp = k.blk;
+      a.st = order_strides(k.e);
+      a.scomp = k.e[0] * k.e[1] * k.e[2] * k.e[3];
       a.expcutoff = cutoff;
       a.rys = rys;
       a.nsplit = L.nsplit;
