@@ -41,10 +41,9 @@ cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int
                                const double* out, const double* dm, int nao, double* A, double* B, cudaStream_t stream,
                                int ni, int nj, int nk, int nl);
 cudaError_t launch_symmetrize(const double* X, double* M, int n, cudaStream_t stream);
-cudaError_t launch_scatter_s8(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
-                              const double* out, double* eri, cudaStream_t stream);
 cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
-                              const double* out, double* eri, int mode, long long nao, cudaStream_t stream);
+                              const double* out, double* eri, int mode, long long nao, int ni, int nj, int nk, int nl,
+                              cudaStream_t stream);
 }
 
 namespace cintx {
@@ -1044,17 +1043,19 @@ int cintx_plan_execute_ao(CintxPlan* p, int aosym, double* eri, int64_t len, voi
     set_error(CINTX_STATUS_ALLOCATION_FAILED, "device allocation for the AO tensor failed");
     return CINTX_STATUS_ALLOCATION_FAILED;
   }
-  cudaMemsetAsync(eri, 0, sizeof(double) * need, stream);  // quartets below the cutoff stay 0
+  // quartets below the cutoff stay 0; a plan of every unique quartet writes every slot
+  const long long np = p->opt->npairs;
+  if (p->stats.nquartets != np * (np + 1) / 2) cudaMemsetAsync(eri, 0, sizeof(double) * need, stream);
   DeviceState* ds;
   ThreadScratch* ts;
   int rc;
   if ((rc = device_state(&ds)) || (rc = thread_scratch(&ts, 0, 0))) return rc;
   auto scatter = [&](const Segment& sg, cudaStream_t st) -> int {
     const QuartetRec* recs = p->d_recs + sg.rec0;
-    const cudaError_t e =
-        aosym == 8 ? launch_scatter_s8(recs, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, eri, st)
-                   : launch_scatter_ao(recs, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, eri, aosym, nao, st);
-    if (e == cudaSuccess) return CINTX_STATUS_SUCCESS;
+    if (launch_scatter_ao(recs, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, eri, aosym, nao, nsph_or_cart(sg.li, p->sph),
+                          nsph_or_cart(sg.lj, p->sph), nsph_or_cart(sg.lk, p->sph), nsph_or_cart(sg.ll, p->sph),
+                          st) == cudaSuccess)
+      return CINTX_STATUS_SUCCESS;
     set_error(CINTX_STATUS_EXECUTION_FAILED, "scatter launch failed");
     return CINTX_STATUS_EXECUTION_FAILED;
   };
