@@ -87,13 +87,21 @@ int ip1_build(const Basis& B, int nsh, const int* shls, int64_t n, bool sph, boo
               int64_t* offsets) {
   const double cutoff = nsh == 4 ? expcutoff_2e(B.env.data()) : expcutoff_3c(B.env.data());
   const double pair_cutoff = opt_mode ? expcutoff_3c(B.env.data()) : cutoff;
-  // (a, b, derivative) -> pair id, packed into one 64-bit key (b may be -1: unit pair)
-  std::unordered_map<uint64_t, int> pair_id;
-  pair_id.reserve(1024);
+  // (a, b, derivative) -> pair id (b may be -1: unit pair).  Lists long enough to meet most pairs of the
+  // basis look them up in a table; short ones (a single call on a large basis) in a hash map.
+  const int nv = B.nvirt;
+  const bool dense = (double)nv * nv <= 16.0 * (double)n;
+  std::vector<int> pair_tab(dense ? (size_t)2 * nv * (nv + 1) : 0, -1);
+  std::unordered_map<uint64_t, int> pair_map;
   auto get_pair = [&](int a, int b, bool deriv) {
-    const uint64_t key = ((uint64_t)(uint32_t)a << 33) | ((uint64_t)(uint32_t)(b + 1) << 1) | (deriv ? 1u : 0u);
-    auto it = pair_id.find(key);
-    if (it != pair_id.end()) return it->second;
+    int* slot;
+    if (dense) {
+      slot = &pair_tab[((size_t)a * (nv + 1) + (b + 1)) * 2 + (deriv ? 1 : 0)];
+    } else {
+      const uint64_t key = ((uint64_t)(uint32_t)a << 33) | ((uint64_t)(uint32_t)(b + 1) << 1) | (deriv ? 1u : 0u);
+      slot = &pair_map.emplace(key, -1).first->second;
+    }
+    if (*slot >= 0) return *slot;
     PairHost ph;
     build_pair(B, a, b, pair_cutoff, ph, deriv || (opt_mode && b >= 0) ? 1 : 0);
     if (deriv) {  // 2 a_i of each primitive pair's i primitive
@@ -105,20 +113,19 @@ int ip1_build(const Basis& B, int nsh, const int* shls, int64_t n, bool sph, boo
     const int id = (int)W.pairs.size();
     W.pairs.push_back(ph.sp);
     W.pair_min_cce.push_back(ph.prims.empty() ? 1e300 : ph.min_cce);
-    pair_id[key] = id;
+    *slot = id;
     return id;
   };
   auto ncomp = [&](int l) { return sph ? 2 * l + 1 : (l + 1) * (l + 2) / 2; };
   // recurrence centre of each (k, l) pair, computed once per pair (pair_base_first loops over the
-  // primitive exponents)
-  std::unordered_map<uint64_t, bool> kfirst;
+  // primitive exponents): -1 not yet, else whether k comes first
+  std::vector<signed char> first_tab(dense ? (size_t)B.nbas * B.nbas : 0, -1);
+  std::unordered_map<uint64_t, signed char> first_map;
   auto centre_first = [&](int k, int l2) {
-    const uint64_t key = ((uint64_t)(uint32_t)k << 32) | (uint32_t)l2;
-    auto it = kfirst.find(key);
-    if (it != kfirst.end()) return it->second;
-    const bool f = pair_base_first(B, k, l2);
-    kfirst.emplace(key, f);
-    return f;
+    signed char& f = dense ? first_tab[(size_t)k * B.nbas + l2]
+                           : first_map.emplace(((uint64_t)(uint32_t)k << 32) | (uint32_t)l2, -1).first->second;
+    if (f < 0) f = pair_base_first(B, k, l2) ? 1 : 0;
+    return f != 0;
   };
   Ip1Work::Group* last = nullptr;  // consecutive tuples mostly share a group
   Ip1Work::Key last_key{};
@@ -128,13 +135,13 @@ int ip1_build(const Basis& B, int nsh, const int* shls, int64_t n, bool sph, boo
     int rs[4] = {s[0], s[1], s[2], nsh == 4 ? s[3] : -1};
     int l[4], nc[4], ne[4];
     for (int a = 0; a < 4; ++a) {
-      if (rs[a] < 0) {
+      if (rs[a] < 0 && (a == 1 || a == 3)) {  // the unit function
         l[a] = 0;
         nc[a] = 1;
         ne[a] = 1;
         continue;
       }
-      if (rs[a] >= B.nbas) {
+      if (rs[a] < 0 || rs[a] >= B.nbas) {
         set_error(CINTX_STATUS_INVALID_INPUT, "shell index out of range in tuple " + std::to_string(q));
         return CINTX_STATUS_INVALID_INPUT;
       }
