@@ -42,7 +42,7 @@ PrimSplit prim_split(int lanes, int most, double resident, double work, long lon
 }
 
 PrimSplit prim_split(int li, int lj, int lk, int ll, double work, long long nrec, double pmax) {
-  const int s = pick_threads(li, lj, lk, ll, variant_acc(0));
+  const int s = default_threads(li, lj, lk, ll);
   if (split_max(s) <= 1) return PrimSplit();
   return prim_split(s, split_max(s), (double)device_sm_count() * 4 * (128 / s), work, nrec, pmax);
 }
@@ -54,27 +54,45 @@ static bool splitcoop_applies(int li, int lj, int lk, int ll, int variant) {
   return variant_splitcoop(variant) && li <= CINTX_LMAX && splitcoop_dims(li, lj, lk, ll, splitcoop_acc(variant)).ok;
 }
 
+// variants that are the default shape for a class (dispatch_lij compiles only the others)
+static bool is_default(int li, int lj, int lk, int ll, bool sph, bool fp32, int variant) {
+  if (!sph || fp32 || variant <= 0 || variant >= kNumVariants) return true;
+  if (variant_splitcoop(variant)) return !splitcoop_applies(li, lj, lk, ll, variant);
+  if (variant_sliced(variant)) return !sliced_ok(li, lj, lk, ll, variant);
+  // one-lane shapes take no register cap
+  return default_threads(li, lj, lk, ll) == 1 &&
+         (variant == 3 || pick_threads(li, lj, lk, ll, variant_acc(variant)) == 1);
+}
+
 int variant_lanes(int li, int lj, int lk, int ll, bool sph, bool fp32, int variant) {
-  if (!sph || fp32 || variant <= 0 || variant >= kNumVariants) variant = 0;
-  if (variant_splitcoop(variant))
-    return splitcoop_applies(li, lj, lk, ll, variant) ? pick_threads(li, lj, lk, ll, splitcoop_acc(variant))
-                                                      : pick_threads(li, lj, lk, ll, variant_acc(0));
-  if (variant_sliced(variant) && !sliced_ok(li, lj, lk, ll, variant)) variant = 0;
+  if (is_default(li, lj, lk, ll, sph, fp32, variant)) return default_threads(li, lj, lk, ll);
+  if (variant_splitcoop(variant)) return pick_threads(li, lj, lk, ll, splitcoop_acc(variant));
   return pick_threads(li, lj, lk, ll, variant_acc(variant)) / variant_passes(variant);
 }
 
 int variant_shape(int li, int lj, int lk, int ll, bool sph, bool fp32, int variant) {
-  if (!sph || fp32 || variant <= 0 || variant >= kNumVariants) variant = 0;
-  if (variant_splitcoop(variant)) {
-    if (!splitcoop_applies(li, lj, lk, ll, variant)) variant = 0;
-    else return (1 << 23) + pick_threads(li, lj, lk, ll, splitcoop_acc(variant)) * 1024 + kSplitCoopRegs;
+  if (is_default(li, lj, lk, ll, sph, fp32, variant)) {
+    const int s = default_threads(li, lj, lk, ll);
+    return s == 1 ? 1 : s * 1024 + variant_regs(0);
   }
-  if (variant_sliced(variant) && !sliced_ok(li, lj, lk, ll, variant)) variant = 0;
+  if (variant_splitcoop(variant))
+    return (1 << 23) + pick_threads(li, lj, lk, ll, splitcoop_acc(variant)) * 1024 + kSplitCoopRegs;
   const int s = pick_threads(li, lj, lk, ll, variant_acc(variant));
-  if (s == 1) return 1;  // one-lane shapes take no register cap
+  if (s == 1) return 1;
   return (variant_sliced(variant) ? 1 << 20 : 0) + (variant_roll(variant) ? 1 << 21 : 0) +
          (variant_passes(variant) > 1 ? 1 << 22 : 0) + s * 1024 +
          variant_regs(variant);
+}
+
+int default_variant(int li, int lj, int lk, int ll) {
+  if (li > CINTX_LMAX || !class_valid(li, lj, lk, ll) || default_threads(li, lj, lk, ll) == 1) return 0;
+  auto lanes = [&](int v) { return sliced_ok(li, lj, lk, ll, v) ? pick_threads(li, lj, lk, ll, variant_acc(v)) : 0; };
+  if (lanes(4) == 2) return 4;
+  if (lanes(5) == 2) return 5;
+  if (lanes(7) > 0) return 7;
+  for (int v : {11, 10})
+    if (splitcoop_applies(li, lj, lk, ll, v)) return v;
+  return 0;
 }
 
 bool class_needs_scratch(int li, int lj, int lk, int ll, bool sph, int variant) {

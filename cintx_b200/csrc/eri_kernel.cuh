@@ -58,6 +58,17 @@ __host__ __device__ constexpr int pick_threads(int li, int lj, int lk, int ll, i
   return s;
 }
 
+// Accumulators per lane of the default shape: classes of at most 48 functions keep the whole block, and
+// with it the whole recurrence, in one lane's registers; larger classes hand out 24 per lane.  (Two lanes
+// of 24 that share their tables in shared memory were 2 to 6 times slower: (20|20) 4.17 -> 0.69 ms,
+// (22|00) 3.18 -> 0.68, (31|00) 10.6 -> 4.4, (30|10) 8.3 -> 3.5 on a 120-atom molecule's largest launches.)
+__host__ __device__ constexpr int default_acc(int li, int lj, int lk, int ll) {
+  return ncart(li) * ncart(lj) * ncart(lk) * ncart(ll) <= 48 ? 48 : 24;
+}
+__host__ __device__ constexpr int default_threads(int li, int lj, int lk, int ll) {
+  return pick_threads(li, lj, lk, ll, default_acc(li, lj, lk, ll));
+}
+
 // Launch-shape variants the autotuner chooses between: the accumulator budget per lane and the
 // register cap of multi-lane shapes (variant 0 is the default shape, used by plans that are not
 // autotuned).  A 255-register cap halves the resident blocks but removes the spills that the
@@ -90,7 +101,8 @@ __host__ __device__ constexpr bool sliced_ok(int li, int lj, int lk, int ll, int
                       3 * (li + 1) * (lj + 1) * (lk + 1) * (ll + 1) <= (v == 4 || v == 8 ? 48 : 72);
 }
 
-template <int LI, int LJ, int LK, int LL, bool SPH, class R = double, int ACC = 24, int REGS = 128,
+template <int LI, int LJ, int LK, int LL, bool SPH, class R = double,
+          int ACC = default_acc(LI, LJ, LK, LL), int REGS = 128,
           bool SLICE = false, bool ROLL = false, int PASSES = 1>
 struct EriShape {
   static constexpr int NR = (LI + LJ + LK + LL) / 2 + 1;
@@ -583,7 +595,8 @@ __device__ __forceinline__ void prim_loop_one_lane(const ShellPair& pij, const S
 // most for S == 1), each evaluating its share of the primitive quartets (split_la); their partial
 // blocks are added before the j, k and l transform stages, which all lanes of the team run.  It is the
 // shape of launches whose longest quartet would otherwise run on long after the others (prim_split).
-template <int LI, int LJ, int LK, int LL, bool SPH, class R = double, int ACC = 24, int REGS = 128,
+template <int LI, int LJ, int LK, int LL, bool SPH, class R = double,
+          int ACC = default_acc(LI, LJ, LK, LL), int REGS = 128,
           bool SLICE = false, bool ROLL = false, int PASSES = 1, bool SPLIT = false>
 __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>::BLOCK,
                                   EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>::MINB)

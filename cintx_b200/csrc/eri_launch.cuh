@@ -45,7 +45,8 @@ __host__ __device__ constexpr int split_max(int s) { return s == 1 ? 32 : (s < 1
 #include "eri_splitcoop.cuh"
 namespace cintx {
 
-template <int LI, int LJ, int LK, int LL, bool SPH, class R = double, int ACC = 24, int REGS = 128,
+template <int LI, int LJ, int LK, int LL, bool SPH, class R = double,
+          int ACC = default_acc(LI, LJ, LK, LL), int REGS = 128,
           bool SLICE = false, bool ROLL = false, int PASSES = 1, bool SPLIT = false>
 cudaError_t launch_eri(const LaunchArgs& a) {
   using SH = EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>;
@@ -99,15 +100,15 @@ cudaError_t dispatch_lij(int lk, int ll, bool sph, const LaunchArgs& a) {
         if (lk == k && ll == l) {
           // variants that give the default shape (lanes, and for multi-lane shapes the register
           // cap) are not compiled separately
-          constexpr int s0 = pick_threads(LI, LJ, k, l, variant_acc(0));
+          constexpr int s0 = default_threads(LI, LJ, k, l);
           constexpr int s1 = pick_threads(LI, LJ, k, l, variant_acc(1));
           constexpr int s2 = pick_threads(LI, LJ, k, l, variant_acc(2));
           // only shapes that differ from the default are instantiated (if constexpr)
           bool done = false;
           if constexpr (split_max(s0) > 1) {
             if (!a.fp32 && a.nsplit > 1) {
-              err = sph ? launch_eri<LI, LJ, k, l, true, double, 24, 128, false, false, 1, true>(a)
-                        : launch_eri<LI, LJ, k, l, false, double, 24, 128, false, false, 1, true>(a);
+              err = sph ? launch_eri<LI, LJ, k, l, true, double, default_acc(LI, LJ, k, l), 128, false, false, 1, true>(a)
+                        : launch_eri<LI, LJ, k, l, false, double, default_acc(LI, LJ, k, l), 128, false, false, 1, true>(a);
               done = true;
             }
           }

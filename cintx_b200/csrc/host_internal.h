@@ -247,5 +247,16 @@ int variant_lanes(int li, int lj, int lk, int ll, bool sph, bool fp32, int varia
 // Distinct launch shape of a variant (lanes and register cap), for telling variants apart.
 int variant_shape(int li, int lj, int lk, int ll, bool sph, bool fp32, int variant);
 constexpr int kLaunchVariants = 12;
+// The variant a spherical FP64 launch starts with when nothing was tuned, by the class's size alone:
+//   at most 48 functions         the default shape, one lane (default_acc);
+//   2 lanes of 32, or else of 48 the sliced shapes with their roots unrolled (4, 5): every lane its own
+//                                recurrences in registers, no barrier per primitive quartet;
+//   up to 4 lanes of 48          the same with the roots rolled (7), tables of at most 72 doubles;
+//   64 lanes or more             split horizontal transfers (11: 24 accumulators per lane, else 10: 12);
+//   the rest                     the default shape.
+// All classes of a 120-atom s/p/d/f molecule, one after another: default shapes 274.7 ms, this rule
+// 202.6, the fastest shape of each class as timed by the autotuner 202.1; 3-centre sweep of 40 atoms 3.84,
+// 2.81 and 2.72 ms.
+int default_variant(int li, int lj, int lk, int ll);
 
 }  // namespace cintx

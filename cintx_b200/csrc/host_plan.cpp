@@ -107,7 +107,7 @@ struct Segment {
   int nranges = 0;
   bool fp32 = false;       // FP32 recurrences (mixed-precision plans)
   double prim_eps = 0;     // primitive Schwarz threshold (tuned plans)
-  int variant = 0;         // launch shape chosen by cintx_plan_autotune (0: default)
+  int variant = 0;         // launch shape: default_variant, or the choice of cintx_plan_autotune
   int nsplit = 1;          // groups sharing each quartet's primitive quartets (prim_split); > 1: default shape
   bool swap = false;       // screened: the tile's records are (col, row) pairs
 };
@@ -515,6 +515,7 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
       p->stride_sets.push_back(order_strides({extent[0], extent[1], extent[2], extent[3]}));
       sg.expcutoff = cutoff;
       sg.rec0 = rec0;
+      if (p->sph) sg.variant = default_variant(k.li, k.lj, k.lk, k.ll);
       ch.segs.push_back(sg);
       seg_work.emplace_back(0.0, 0.0);
       seg_extent = extent;
@@ -1807,7 +1808,8 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
             const long long q0 = part ? rs : r0, q1 = part ? seg_end[g] : rs;
             if (q1 <= q0) continue;
             ok = launch_class(la, lb, la, lb, true, d_recs + q0, (int)(q1 - q0), o->d_pairs, o->d_prims, d_out, one_stride(st),
-                              ecut, ds->rys, ts->stream, false, 0.0, 0, nullptr, nullptr, part ? 1 : ps.ns) ==
+                              ecut, ds->rys, ts->stream, false, 0.0, default_variant(la, lb, la, lb), nullptr, nullptr,
+                              part ? 1 : ps.ns) ==
                  cudaSuccess;
             ts->launches++;
           }
@@ -2100,6 +2102,7 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
       m.prim_eps = p0.prim_eps;
       m.swap = p0.swap;
       m.nsplit = nsplit;
+      if (p->sph && !m.fp32) m.variant = default_variant(m.li, m.lj, m.lk, m.ll);
       m.rec0 = rec;
       m.out_off = 0;
       m.range0 = (int)p->ranges.size();
