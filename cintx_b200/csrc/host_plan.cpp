@@ -37,12 +37,12 @@ cudaError_t launch_prim_x(const QuartetRec* recs, long long nrec, const ShellPai
                           const long long* pbase, double* xout, cudaStream_t stream);
 cudaError_t launch_block_absmax_sqrt(const QuartetRec* recs, long long nrec, const double* out, const long long* len,
                                      double* q, cudaStream_t stream);
-cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
-                               const double* out, const double* dm, int nao, double* A, double* B, cudaStream_t stream,
+cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
+                               const double* dm, int nao, double* A, double* B, cudaStream_t stream,
                                int ni, int nj, int nk, int nl);
 cudaError_t launch_symmetrize(const double* X, double* M, int n, cudaStream_t stream);
-cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
-                              const double* out, double* eri, int mode, long long nao, int ni, int nj, int nk, int nl,
+cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
+                              double* eri, int mode, long long nao, int ni, int nj, int nk, int nl,
                               cudaStream_t stream);
 }
 
@@ -184,9 +184,8 @@ struct CintxPlan {
   // quartet, and per record its base (doubles) in d_rootbuf
   double* d_rootbuf = nullptr;
   long long* d_rootbase = nullptr;
-  // J/K builds (cintx_plan_jk): shells of each regular pair, AO offsets, accumulators, chunk ring
-  int2* d_psh = nullptr;
-  int* d_aoloc = nullptr;
+  // J/K builds (cintx_plan_jk): first functions of each regular pair, accumulators, chunk ring
+  int2* d_pao = nullptr;
   double* d_jkacc = nullptr;
   long long jk_cap = 0;
   cudaEvent_t ev_done[2] = {nullptr, nullptr};
@@ -223,6 +222,10 @@ void free_plan_device(CintxPlan* p) {
   if (p->d_rootbase) cudaFree(p->d_rootbase);
   p->d_rootbuf = nullptr;
   p->d_rootbase = nullptr;
+  if (p->d_pao) cudaFree(p->d_pao);
+  if (p->d_jkacc) cudaFree(p->d_jkacc);
+  p->d_pao = nullptr;
+  p->d_jkacc = nullptr;
   for (int b = 0; b < 2; ++b) {
     if (p->ev_done[b]) cudaEventDestroy(p->ev_done[b]);
     if (p->ev_free[b]) cudaEventDestroy(p->ev_free[b]);
@@ -986,19 +989,19 @@ int cintx_plan_use_learned_roots(CintxPlan* p, const float* params, int64_t* nfa
   return CINTX_STATUS_SUCCESS;
 }
 
-// Device copies of each regular pair's shells and of the AO offsets (cached in the plan).
+// Device table of each regular pair's first functions (cached in the plan): block axes 0 and 1 of a pair
+// are its shells in reported order (the layout screened plans write); the second entry's sign bit marks a
+// pair of one shell (plan_kernels.cu).
 static bool ao_maps(CintxPlan* p, const std::vector<int>& aoloc) {
-  if (p->d_psh) return true;
+  if (p->d_pao) return true;
   const Opt* o = p->opt;
-  // block axes 0 and 1 of a pair: its shells in reported order (the layout screened plans write)
-  std::vector<int2> psh(o->npairs);
-  for (int id = 0; id < o->npairs; ++id) psh[id] = reported_shells(o, id);
-  bool ok = cudaMalloc(&p->d_psh, sizeof(int2) * std::max(o->npairs, 1)) == cudaSuccess &&
-            cudaMalloc(&p->d_aoloc, sizeof(int) * aoloc.size()) == cudaSuccess;
-  if (ok) {
-    cudaMemcpy(p->d_psh, psh.data(), sizeof(int2) * psh.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(p->d_aoloc, aoloc.data(), sizeof(int) * aoloc.size(), cudaMemcpyHostToDevice);
+  std::vector<int2> pao(o->npairs);
+  for (int id = 0; id < o->npairs; ++id) {
+    const int2 sh = reported_shells(o, id);
+    pao[id] = make_int2(aoloc[sh.x], aoloc[sh.y] | (sh.x == sh.y ? (int)0x80000000u : 0));
   }
+  bool ok = cudaMalloc(&p->d_pao, sizeof(int2) * std::max(o->npairs, 1)) == cudaSuccess;
+  if (ok) cudaMemcpy(p->d_pao, pao.data(), sizeof(int2) * pao.size(), cudaMemcpyHostToDevice);
   return ok;
 }
 
@@ -1053,7 +1056,7 @@ int cintx_plan_execute_ao(CintxPlan* p, int aosym, double* eri, int64_t len, voi
   if ((rc = device_state(&ds)) || (rc = thread_scratch(&ts, 0, 0))) return rc;
   auto scatter = [&](const Segment& sg, cudaStream_t st) -> int {
     const QuartetRec* recs = p->d_recs + sg.rec0;
-    if (launch_scatter_ao(recs, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, eri, aosym, nao, nsph_or_cart(sg.li, p->sph),
+    if (launch_scatter_ao(recs, sg.nrec, p->d_pao, p->d_stage, eri, aosym, nao, nsph_or_cart(sg.li, p->sph),
                           nsph_or_cart(sg.lj, p->sph), nsph_or_cart(sg.lk, p->sph), nsph_or_cart(sg.ll, p->sph),
                           st) == cudaSuccess)
       return CINTX_STATUS_SUCCESS;
@@ -1115,7 +1118,7 @@ int cintx_plan_jk(CintxPlan* p, const double* dm, int nao, double* vj, double* v
   int rc;
   if ((rc = device_state(&ds)) || (rc = thread_scratch(&ts, 0, 0))) return rc;
   auto contract = [&](const Segment& sg, cudaStream_t st) -> int {
-    if (launch_jk_contract(p->d_recs + sg.rec0, sg.nrec, p->d_psh, p->d_aoloc, p->d_stage, dm, nao, A, Bk, st,
+    if (launch_jk_contract(p->d_recs + sg.rec0, sg.nrec, p->d_pao, p->d_stage, dm, nao, A, Bk, st,
                            nsph_or_cart(sg.li, p->sph), nsph_or_cart(sg.lj, p->sph), nsph_or_cart(sg.lk, p->sph),
                            nsph_or_cart(sg.ll, p->sph)) == cudaSuccess)
       return CINTX_STATUS_SUCCESS;

@@ -114,6 +114,11 @@ __global__ void block_absmax_sqrt_kernel(const QuartetRec* __restrict__ recs, lo
   }
 }
 
+// The AO table of a plan's pairs: first functions of the pair's two shells (block axes 0 and 1), the
+// second one's sign bit set where both are one shell (those blocks hold every element twice).
+__device__ __forceinline__ int pair_ao(const int2& p) { return p.y & 0x7fffffff; }
+__device__ __forceinline__ double pair_weight(const int2& p) { return p.y < 0 ? 0.5 : 1.0; }
+
 // Coulomb/exchange contraction of one chunk of a unique-quartet sweep (a >= b, c >= d, ab >= cd):
 // one warp per quartet block v[i + ni*(j + nj*(k + nk*l))] (shells a, b, c, d), with the 8-fold
 // permutational symmetry of real integrals and a symmetric density D (row-major nao x nao):
@@ -122,19 +127,16 @@ __global__ void block_absmax_sqrt_kernel(const QuartetRec* __restrict__ recs, lo
 //   B[i,l] += s sum_jk v D[j,k],  B[j,l] += s sum_ik v D[i,k]               (K = B + B^T)
 // with s = 1/2 for each of a == b, c == d, (ab) == (cd) (those blocks hold every element twice).
 // Each (row, column) pair of a block reduces its sum first and adds it with one atomic.
-__global__ void jk_contract_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ psh,
-                                   const int* __restrict__ aoloc, const double* __restrict__ out,
-                                   const double* __restrict__ dm, int nao, double* __restrict__ A,
-                                   double* __restrict__ B) {
+__global__ void jk_contract_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
+                                   const double* __restrict__ out, const double* __restrict__ dm, int nao,
+                                   double* __restrict__ A, double* __restrict__ B, int ni, int nj, int nk, int nl) {
   const int lane = threadIdx.x & 31;
   for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < nrec;
        r += ((long long)gridDim.x * blockDim.x) >> 5) {
     const QuartetRec rec = recs[r];
-    const int2 ab = psh[rec.pij], cd = psh[rec.pkl];
-    const int i0 = aoloc[ab.x], j0 = aoloc[ab.y], k0 = aoloc[cd.x], l0 = aoloc[cd.y];
-    const int ni = aoloc[ab.x + 1] - i0, nj = aoloc[ab.y + 1] - j0;
-    const int nk = aoloc[cd.x + 1] - k0, nl = aoloc[cd.y + 1] - l0;
-    const double s = (ab.x == ab.y ? 0.5 : 1.0) * (cd.x == cd.y ? 0.5 : 1.0) * (rec.pij == rec.pkl ? 0.5 : 1.0);
+    const int2 ab = pao[rec.pij], cd = pao[rec.pkl];
+    const int i0 = ab.x, j0 = pair_ao(ab), k0 = cd.x, l0 = pair_ao(cd);
+    const double s = pair_weight(ab) * pair_weight(cd) * (rec.pij == rec.pkl ? 0.5 : 1.0);
     const double* v = out + rec.out;
     const int sj = ni, sk = ni * nj, sl = ni * nj * nk;
     if (A) {
@@ -205,9 +207,8 @@ __device__ __forceinline__ unsigned small_div(unsigned e, const SmallDiv& v) { r
 // and scatter, beside the sweep itself: s8 of 24 atoms (2.0 GB) 863 -> 632 us, s4 of 18 (1.1 GB) 580 -> 496,
 // s1 of 14 (1.9 GB, 254 of it the clearing) 980 -> 947.
 template <int MODE>
-__global__ void scatter_ao_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ psh,
-                                  const int* __restrict__ aoloc, const double* __restrict__ out,
-                                  double* __restrict__ eri, long long nao, SmallDiv ni, SmallDiv nj, SmallDiv nk,
+__global__ void scatter_ao_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
+                                  const double* __restrict__ out, double* __restrict__ eri, long long nao, SmallDiv ni, SmallDiv nj, SmallDiv nk,
                                   SmallDiv nl, int G) {
   const int g = threadIdx.x & (G - 1);
   const long long npair = nao * (nao + 1) / 2, n2 = nao * nao;
@@ -216,8 +217,8 @@ __global__ void scatter_ao_kernel(const QuartetRec* __restrict__ recs, long long
   const long long ngroups = (long long)gridDim.x * blockDim.x / G;
   for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G; r < nrec; r += ngroups) {
     const QuartetRec rec = recs[r];
-    const int2 ab = psh[rec.pij], cd = psh[rec.pkl];
-    const long long i0 = aoloc[ab.x], j0 = aoloc[ab.y], k0 = aoloc[cd.x], l0 = aoloc[cd.y];
+    const int2 ab = pao[rec.pij], cd = pao[rec.pkl];
+    const long long i0 = ab.x, j0 = pair_ao(ab), k0 = cd.x, l0 = pair_ao(cd);
     const double* v = out + rec.out;
     if constexpr (MODE == 1) {
       for (unsigned e = g; e < n; e += G) {  // l fastest, then k, j, i
@@ -255,7 +256,7 @@ __global__ void scatter_ao_kernel(const QuartetRec* __restrict__ recs, long long
     } else {
       // an AO pair's packed index runs along its smaller function: fastest the smaller shell of each side
       // (a block of a diagonal pair, which reaches slots twice, in its own order in both: the last one stays)
-      const bool twice = ab.x == ab.y || cd.x == cd.y || rec.pij == rec.pkl;
+      const bool twice = ab.y < 0 || cd.y < 0 || rec.pij == rec.pkl;
       const bool klow = twice || k0 < l0, ilow = twice || i0 < j0;
       const SmallDiv f1 = klow ? nk : nl, f2 = klow ? nl : nk, f3 = ilow ? ni : nj, f4 = ilow ? nj : ni;
       for (int pass = 0; pass < (MODE == 4 ? 2 : 1); ++pass) {
@@ -335,8 +336,8 @@ __device__ __forceinline__ void halving_sum(double (&p)[N], int G, unsigned mask
 
 template <int NK, int NL>
 __global__ void __launch_bounds__(32 * kJkWarps)
-    jk_contract_group_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ psh,
-                             const int* __restrict__ aoloc, const double* __restrict__ out,
+    jk_contract_group_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
+                             const double* __restrict__ out,
                              const double* __restrict__ dm, int nao, double* __restrict__ A, double* __restrict__ B,
                              int ni, int nj, int G, int run) {
   constexpr int NP = NK <= 1 ? 1 : NK <= 2 ? 2 : NK <= 4 ? 4 : NK <= 8 ? 8 : 16;
@@ -356,21 +357,27 @@ __global__ void __launch_bounds__(32 * kJkWarps)
     int cur = -1;  // the (ij) pair whose A[i,j] sums s_aij holds
     int i0 = 0, j0 = 0;
     double sij = 0;
+    QuartetRec next = recs[base];
+    int2 next_cd = pao[next.pkl];
     for (long long r = base; r < rend; ++r) {
-      const QuartetRec rec = recs[r];
-      const int2 cd = psh[rec.pkl];
-      const int k0 = aoloc[cd.x], l0 = aoloc[cd.y];
+      const QuartetRec rec = next;
+      const int2 cd = next_cd;
+      if (r + 1 < rend) {  // on its way while this quartet is contracted
+        next = recs[r + 1];
+        next_cd = pao[next.pkl];
+      }
+      const int k0 = cd.x, l0 = pair_ao(cd);
       if (rec.pij != cur) {
         if (cur >= 0 && A)
           for (int e = g; e < nij; e += G) atomicAdd(A + (size_t)(i0 + e % ni) * nao + j0 + e / ni, s_aij[e]);
-        const int2 ab = psh[rec.pij];
-        i0 = aoloc[ab.x];
-        j0 = aoloc[ab.y];
-        sij = ab.x == ab.y ? 0.5 : 1.0;
+        const int2 ab = pao[rec.pij];
+        i0 = ab.x;
+        j0 = pair_ao(ab);
+        sij = pair_weight(ab);
         cur = rec.pij;
         for (int e = g; e < nij; e += G) s_aij[e] = 0.0;
       }
-      const double s = sij * (cd.x == cd.y ? 0.5 : 1.0) * (rec.pij == rec.pkl ? 0.5 : 1.0);
+      const double s = sij * pair_weight(cd) * (rec.pij == rec.pkl ? 0.5 : 1.0);
       for (int e = g; e < NK * NL; e += G) {
         s_dkl[e] = dm[(size_t)(k0 + e % NK) * nao + l0 + e / NK];
         s_akl[e] = 0.0;
@@ -490,8 +497,8 @@ cudaError_t launch_block_absmax_sqrt(const QuartetRec* recs, long long nrec, con
 }
 
 template <int NK, int NL>
-static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
-                                   const double* out, const double* dm, int nao, double* A, double* B,
+static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
+                                   const double* dm, int nao, double* A, double* B,
                                    cudaStream_t stream, int ni, int nj) {
   int G = 1;
   while (G < 32 && G < ni * nj) G *= 2;
@@ -506,19 +513,19 @@ static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const
   const long long per_block = 32LL * kJkWarps / G * run;
   long long blocks = (nrec + per_block - 1) / per_block;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
-  kern<<<(unsigned)blocks, 32 * kJkWarps, smem, stream>>>(recs, nrec, psh, aoloc, out, dm, nao, A, B, ni, nj, G, run);
+  kern<<<(unsigned)blocks, 32 * kJkWarps, smem, stream>>>(recs, nrec, pao, out, dm, nao, A, B, ni, nj, G, run);
   return cudaGetLastError();
 }
 
 // One class segment, blocks ni x nj x nk x nl.  Ket extents up to 10 have their own kernel (sph 1..9,
 // cart 1..10); cartesian g kets (15 functions: the sums of one lane no longer fit registers) keep the
 // general kernel.
-cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
-                               const double* out, const double* dm, int nao, double* A, double* B, cudaStream_t stream,
+cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
+                               const double* dm, int nao, double* A, double* B, cudaStream_t stream,
                                int ni, int nj, int nk, int nl) {
   if (nrec <= 0) return cudaSuccess;
 #define CINTX_JK(K, L) \
-  if (nk == K && nl == L) return launch_jk_group<K, L>(recs, nrec, psh, aoloc, out, dm, nao, A, B, stream, ni, nj);
+  if (nk == K && nl == L) return launch_jk_group<K, L>(recs, nrec, pao, out, dm, nao, A, B, stream, ni, nj);
   if (jk_group_doubles(ni * nj, nk, nl) * sizeof(double) * kJkWarps <= 200 * 1024) {
     CINTX_JK(1, 1) CINTX_JK(3, 1) CINTX_JK(3, 3)
     CINTX_JK(5, 1) CINTX_JK(5, 3) CINTX_JK(5, 5)
@@ -530,12 +537,12 @@ cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int
 #undef CINTX_JK
   long long blocks = (nrec * 32 + 255) / 256;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
-  jk_contract_kernel<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, psh, aoloc, out, dm, nao, A, B);
+  jk_contract_kernel<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, pao, out, dm, nao, A, B, ni, nj, nk, nl);
   return cudaGetLastError();
 }
 
-cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2* psh, const int* aoloc,
-                              const double* out, double* eri, int mode, long long nao, int ni, int nj, int nk, int nl,
+cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
+                              double* eri, int mode, long long nao, int ni, int nj, int nk, int nl,
                               cudaStream_t stream) {
   if (nrec <= 0) return cudaSuccess;
   auto div = [](int d) { return SmallDiv{(unsigned)d, d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d)}; };
@@ -544,7 +551,7 @@ cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2
   long long blocks = (nrec * G + 255) / 256;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
   auto kern = mode == 1 ? scatter_ao_kernel<1> : (mode == 4 ? scatter_ao_kernel<4> : scatter_ao_kernel<8>);
-  kern<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, psh, aoloc, out, eri, nao, div(ni), div(nj), div(nk), div(nl),
+  kern<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, pao, out, eri, nao, div(ni), div(nj), div(nk), div(nl),
                                              G);
   return cudaGetLastError();
 }
