@@ -52,7 +52,7 @@ __host__ __device__ inline long long rec_offset(const QuartetRec& r) { return r.
 __host__ __device__ inline int rec_strides(const QuartetRec& r) { return (int)((unsigned long long)r.out >> 56); }
 
 // A contiguous run [t0, t1) of one screened tile's row-major quartet numbering, generating
-// records rec_off.. of a merged class segment whose blocks start at out_off (doubles).
+// records rec_off.. of its chunk, whose blocks start at out_off (doubles).
 struct __align__(16) GenRange {
   const int* rows;
   const int* cols;

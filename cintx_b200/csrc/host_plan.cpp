@@ -31,7 +31,7 @@ namespace cintx {
 cudaError_t launch_gen_tile(const int* rows, const int* cols, const long long* row_prefix, int nrows,
                             long long t0, long long t1, long long nout, long long out_base, QuartetRec* recs,
                             cudaStream_t stream);
-cudaError_t launch_gen_ranges(const GenRange* ranges, int nranges, long long nrec, QuartetRec* recs,
+cudaError_t launch_gen_ranges(const GenRange* ranges, int nranges, long long rbegin, long long rend, QuartetRec* recs,
                               cudaStream_t stream);
 cudaError_t launch_prim_x(const QuartetRec* recs, long long nrec, const ShellPair* pairs, const PrimPair* prims,
                           const long long* pbase, double* xout, cudaStream_t stream);
@@ -601,20 +601,32 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
   return CINTX_STATUS_SUCCESS;
 }
 
+// Writes the records of a screened chunk's segments [s0, s1) on `stream`.
+static int gen_records(CintxPlan* p, const Segment* s0, const Segment* s1, cudaStream_t stream, ThreadScratch* ts) {
+  if (s0 == s1 || s0->tile != -2) return CINTX_STATUS_SUCCESS;
+  const Segment& last = s1[-1];
+  const cudaError_t e = launch_gen_ranges(p->d_ranges + s0->range0, last.range0 + last.nranges - s0->range0, s0->rec0,
+                                          last.rec0 + last.nrec, p->d_recs, stream);
+  if (e != cudaSuccess) {
+    set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("quartet generation failed: ") + cudaGetErrorString(e));
+    return CINTX_STATUS_EXECUTION_FAILED;
+  }
+  ts->launches++;
+  return CINTX_STATUS_SUCCESS;
+}
+
+// Runs one segment's class kernel; gen: its records are written first (else they are there already).
 static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStream_t stream, DeviceState* ds,
-                       ThreadScratch* ts) {
+                       ThreadScratch* ts, bool gen) {
   const Opt* o = p->opt;
   const QuartetRec* recs;
   long long nrec;
   if (sg.tile == -2) {
-    QuartetRec* dst = p->d_recs + sg.rec0;
-    cudaError_t e = launch_gen_ranges(p->d_ranges + sg.range0, sg.nranges, sg.nrec, dst, stream);
-    if (e != cudaSuccess) {
-      set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("quartet generation failed: ") + cudaGetErrorString(e));
-      return CINTX_STATUS_EXECUTION_FAILED;
+    if (gen) {
+      const int rc = gen_records(p, &sg, &sg + 1, stream, ts);
+      if (rc) return rc;
     }
-    ts->launches++;
-    recs = dst;
+    recs = p->d_recs + sg.rec0;
     nrec = sg.nrec;
   } else if (sg.tile < 0) {
     recs = p->d_recs + sg.rec0;
@@ -662,8 +674,10 @@ static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStr
 constexpr double kForkFlops = 4e9;
 static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_t stream, DeviceState* ds,
                      ThreadScratch* ts, const std::function<int(const Segment&, cudaStream_t)>& after) {
-  int rc = CINTX_STATUS_SUCCESS;
   const int n = (int)ch.segs.size();
+  // one launch writes the whole chunk's records, ahead of the fork
+  int rc = gen_records(p, ch.segs.data(), ch.segs.data() + n, stream, ts);
+  if (rc) return rc;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   SideStreams* side = nullptr;
   double total = 0;
@@ -674,7 +688,7 @@ static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_
   }
   if (!side) {
     for (const Segment& sg : ch.segs) {
-      if ((rc = run_segment(p, sg, out_dev, stream, ds, ts))) return rc;
+      if ((rc = run_segment(p, sg, out_dev, stream, ds, ts, false))) return rc;
       if (after && (rc = after(sg, stream))) return rc;
     }
     return CINTX_STATUS_SUCCESS;
@@ -689,7 +703,7 @@ static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_
     cudaStream_t st =
         fork.next(sg.flops + 3e7, class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant));
     if (fork.error() != cudaSuccess) break;
-    if ((rc = run_segment(p, sg, out_dev, st, ds, ts)) || (after && (rc = after(sg, st)))) break;
+    if ((rc = run_segment(p, sg, out_dev, st, ds, ts, false)) || (after && (rc = after(sg, st)))) break;
   }
   const cudaError_t e = fork.join();
   give_side_streams(ds->dev, side);
@@ -741,7 +755,7 @@ int cintx_plan_execute_segment(CintxPlan* p, int64_t chunk, int seg, double* out
     set_error(CINTX_STATUS_INVALID_INPUT, "chunk or segment index out of range");
     return CINTX_STATUS_INVALID_INPUT;
   }
-  return run_segment(p, p->chunks[chunk].segs[seg], out_dev, stream, ds, ts);
+  return run_segment(p, p->chunks[chunk].segs[seg], out_dev, stream, ds, ts, true);
 }
 
 int cintx_plan_execute_host(CintxPlan* p, int64_t chunk, double* out_host) {
@@ -1299,9 +1313,9 @@ int cintx_plan_autotune(CintxPlan* p, int64_t chunk, double* out_dev, void* stre
       if (!scratch0 && class_needs_scratch(sg0.li, sg0.lj, sg0.lk, sg0.ll, p->sph, v)) continue;
       Segment sg = sg0;
       sg.variant = v;
-      if ((rc = run_segment(p, sg, out_dev, stream, ds, ts))) break;  // warm-up
+      if ((rc = run_segment(p, sg, out_dev, stream, ds, ts, true))) break;  // warm-up
       cudaEventRecord(e0, stream);
-      for (int r = 0; r < reps && !rc; ++r) rc = run_segment(p, sg, out_dev, stream, ds, ts);
+      for (int r = 0; r < reps && !rc; ++r) rc = run_segment(p, sg, out_dev, stream, ds, ts, false);
       cudaEventRecord(e1, stream);
       if (rc) break;
       if (cudaEventSynchronize(e1) != cudaSuccess) {
@@ -1498,6 +1512,7 @@ int cintx_plan_graph_build(CintxPlan* p, const int64_t* chunks, int64_t n, doubl
   const int64_t l0 = ts->launches;
   for (int64_t c : list) {
     const Chunk& ch = p->chunks[c];
+    rc = gen_records(p, ch.segs.data(), ch.segs.data() + ch.segs.size(), origin, ts);
     cudaEventRecord(p->events[0], origin);
     for (int b = 1; b < nbranch; ++b) cudaStreamWaitEvent(p->branches[b], p->events[0], 0);
     // longest-first assignment of class segments to branches
@@ -1508,7 +1523,7 @@ int cintx_plan_graph_build(CintxPlan* p, const int64_t* chunks, int64_t n, doubl
     for (int i : idx) {
       const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
       load[b] += ch.segs[i].flops + 1.0;
-      if ((rc = run_segment(p, ch.segs[i], out_dev, p->branches[b], ds, ts))) {
+      if (rc || (rc = run_segment(p, ch.segs[i], out_dev, p->branches[b], ds, ts, false))) {
         cudaGraph_t g;
         cudaStreamEndCapture(origin, &g);
         if (g) cudaGraphDestroy(g);
@@ -2121,7 +2136,7 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
         g.colstart = t.d_colstart;
         g.t0 = pc.t0;
         g.t1 = pc.t1;
-        g.rec_off = m.nrec;
+        g.rec_off = m.rec0 + m.nrec;
         g.out_off = pc.out_off;
         g.nout = pc.nout;
         p->ranges.push_back(g);
