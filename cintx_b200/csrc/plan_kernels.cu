@@ -154,6 +154,16 @@ __global__ void block_absmax_sqrt_kernel(const QuartetRec* __restrict__ recs, lo
   }
 }
 
+// Division of a small non-negative number by a block extent: e / d for e < 2^16, d <= 15 (the error of
+// the reciprocal, e (m d - 2^32) / 2^32 < e / 2^28, stays under 1 / d).
+struct SmallDiv {
+  unsigned d, m;  // m = ceil(2^32 / d), 0 for d == 1
+};
+static SmallDiv small_divisor(int d) {
+  return SmallDiv{(unsigned)d, d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d)};
+}
+__device__ __forceinline__ unsigned small_div(unsigned e, const SmallDiv& v) { return v.m ? __umulhi(e, v.m) : e; }
+
 // The AO table of a plan's pairs: first functions of the pair's two shells (block axes 0 and 1), the
 // second one's sign bit set where both are one shell (those blocks hold every element twice).
 __device__ __forceinline__ int pair_ao(const int2& p) { return p.y & 0x7fffffff; }
@@ -227,12 +237,6 @@ __global__ void jk_contract_kernel(const QuartetRec* __restrict__ recs, long lon
     }
   }
 }
-
-// Division of a small non-negative number by a block extent: e / d for e < 2^16, d <= 15.
-struct SmallDiv {
-  unsigned d, m;  // m = ceil(2^32 / d), 0 for d == 1
-};
-__device__ __forceinline__ unsigned small_div(unsigned e, const SmallDiv& v) { return v.m ? __umulhi(e, v.m) : e; }
 
 // Scatters a class segment (blocks ni x nj x nk x nl) of a unique-quartet sweep into an AO tensor, G lanes
 // (the power of two from the block size up, at most a warp) per quartet block:
@@ -379,11 +383,11 @@ __global__ void __launch_bounds__(32 * kJkWarps)
     jk_contract_group_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
                              const double* __restrict__ out,
                              const double* __restrict__ dm, int nao, double* __restrict__ A, double* __restrict__ B,
-                             int ni, int nj, int G, int run) {
+                             SmallDiv di_, SmallDiv dj_, int G, int run) {
   constexpr int NP = NK <= 1 ? 1 : NK <= 2 ? 2 : NK <= 4 ? 4 : NK <= 8 ? 8 : 16;
   constexpr int NKL = NK + NL;
   extern __shared__ double sm[];
-  const int nij = ni * nj;
+  const int ni = (int)di_.d, nj = (int)dj_.d, nij = ni * nj;
   const int lane = threadIdx.x & 31, g = lane & (G - 1);
   const unsigned mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
   double* s_dkl = sm + (size_t)(threadIdx.x / G) * jk_group_doubles(nij, NK, NL);
@@ -409,7 +413,10 @@ __global__ void __launch_bounds__(32 * kJkWarps)
       const int k0 = cd.x, l0 = pair_ao(cd);
       if (rec.pij != cur) {
         if (cur >= 0 && A)
-          for (int e = g; e < nij; e += G) atomicAdd(A + (size_t)(i0 + e % ni) * nao + j0 + e / ni, s_aij[e]);
+          for (int e = g; e < nij; e += G) {
+            const int j = (int)small_div(e, di_);
+            atomicAdd(A + (size_t)(i0 + e - j * ni) * nao + j0 + j, s_aij[e]);
+          }
         const int2 ab = pao[rec.pij];
         i0 = ab.x;
         j0 = pair_ao(ab);
@@ -426,7 +433,7 @@ __global__ void __launch_bounds__(32 * kJkWarps)
       for (int ij0 = 0; ij0 < nij; ij0 += G) {
         const int ij = ij0 + g;
         const bool on = ij < nij;
-        const int i = on ? ij % ni : 0, j = on ? ij / ni : 0;
+        const int j = on ? (int)small_div(ij, di_) : 0, i = on ? ij - j * ni : 0;
         const double* v = out + rec.out + (on ? ij : 0);
         const double* di = dm + (size_t)(i0 + i) * nao;
         const double* dj = dm + (size_t)(j0 + j) * nao;
@@ -486,14 +493,14 @@ __global__ void __launch_bounds__(32 * kJkWarps)
           atomicAdd(A + (size_t)(k0 + e % NK) * nao + l0 + e / NK, 2.0 * s * s_akl[e]);
       if (B) {
         for (int e = g; e < ni * NKL; e += G) {  // B[i, k or l]: sums over j
-          const int i = e % ni, c = e / ni;
+          const int c = (int)small_div(e, di_), i = e - c * ni;
           const double* x = s_t + c * nij + i;
           double sum = 0.0;
           for (int j = 0; j < nj; ++j) sum += x[ni * j];
           atomicAdd(B + (size_t)(i0 + i) * nao + (c < NK ? k0 + c : l0 + c - NK), s * sum);
         }
         for (int e = g; e < nj * NKL; e += G) {  // B[j, k or l]: sums over i
-          const int j = e % nj, c = e / nj;
+          const int c = (int)small_div(e, dj_), j = e - c * nj;
           const double* x = s_t + (NKL + c) * nij + ni * j;
           double sum = 0.0;
           for (int i = 0; i < ni; ++i) sum += x[i];
@@ -503,7 +510,10 @@ __global__ void __launch_bounds__(32 * kJkWarps)
       __syncwarp(mask);
     }
     if (cur >= 0 && A)
-      for (int e = g; e < nij; e += G) atomicAdd(A + (size_t)(i0 + e % ni) * nao + j0 + e / ni, s_aij[e]);
+      for (int e = g; e < nij; e += G) {
+        const int j = (int)small_div(e, di_);
+        atomicAdd(A + (size_t)(i0 + e - j * ni) * nao + j0 + j, s_aij[e]);
+      }
     __syncwarp(mask);
   }
 }
@@ -553,7 +563,8 @@ static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const
   const long long per_block = 32LL * kJkWarps / G * run;
   long long blocks = (nrec + per_block - 1) / per_block;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
-  kern<<<(unsigned)blocks, 32 * kJkWarps, smem, stream>>>(recs, nrec, pao, out, dm, nao, A, B, ni, nj, G, run);
+  kern<<<(unsigned)blocks, 32 * kJkWarps, smem, stream>>>(recs, nrec, pao, out, dm, nao, A, B, small_divisor(ni),
+                                                          small_divisor(nj), G, run);
   return cudaGetLastError();
 }
 
@@ -585,13 +596,13 @@ cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2
                               double* eri, int mode, long long nao, int ni, int nj, int nk, int nl,
                               cudaStream_t stream) {
   if (nrec <= 0) return cudaSuccess;
-  auto div = [](int d) { return SmallDiv{(unsigned)d, d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d)}; };
   int G = 1;
   while (G < 32 && G < ni * nj * nk * nl) G *= 2;
   long long blocks = (nrec * G + 255) / 256;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
   auto kern = mode == 1 ? scatter_ao_kernel<1> : (mode == 4 ? scatter_ao_kernel<4> : scatter_ao_kernel<8>);
-  kern<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, pao, out, eri, nao, div(ni), div(nj), div(nk), div(nl),
+  kern<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, pao, out, eri, nao, small_divisor(ni), small_divisor(nj), small_divisor(nk),
+                                             small_divisor(nl),
                                              G);
   return cudaGetLastError();
 }
