@@ -30,14 +30,24 @@ cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const Quartet
   return dispatch_eri(li, lj, lk, ll, sph, a);
 }
 
+constexpr double kSplitLarge = 1024;
+
 PrimSplit prim_split(int lanes, int most, double resident, double work, long long nrec, double pmax) {
   PrimSplit r;
   if (most <= 1 || nrec <= 0) return r;
   const double share = std::max(work / resident, lanes == 1 ? 16.0 : 4.0);
-  if (pmax < 2 * share) return r;
+  if (pmax < 2 * share) {
+    if (lanes == 1 && pmax >= kSplitLarge) {
+      r.ns = 8;
+      r.pmin = kSplitLarge;
+    }
+    return r;
+  }
   r.ns = 2;
   while (r.ns < most && r.ns * share < pmax) r.ns *= 2;
+  if (lanes == 1 && r.ns == 64) r.ns = 32;  // one-lane teams: at most a warp, or a block
   r.pmin = (double)nrec * r.ns <= 2 * resident ? 0 : 2 * share;
+  if (lanes == 1 && r.pmin > kSplitLarge) r.pmin = kSplitLarge;
   return r;
 }
 

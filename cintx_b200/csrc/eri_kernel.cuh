@@ -591,8 +591,8 @@ __device__ __forceinline__ void prim_loop_one_lane(const ShellPair& pij, const S
   }
 }
 
-// SPLIT: a quartet is shared by a team of nsplit groups (a power of two, nsplit * S <= BLOCK, one warp at
-// most for S == 1), each evaluating its share of the primitive quartets (split_la); their partial
+// SPLIT: a quartet is shared by a team of nsplit groups (a power of two, nsplit * S <= BLOCK; for S == 1
+// at most a warp, or the whole block), each evaluating its share of the primitive quartets (split_la); their partial
 // blocks are added before the j, k and l transform stages, which all lanes of the team run.  It is the
 // shape of launches whose longest quartet would otherwise run on long after the others (prim_split).
 template <int LI, int LJ, int LK, int LL, bool SPH, class R = double,
@@ -677,14 +677,35 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
     if constexpr (S == 1) {
       prim_loop_one_lane<LI, LJ, LK, LL, SH, R>(pij, pkl, prims, rys, SH::STAGE_TABLE ? smem : nullptr, expcutoff,
                                                 prim_eps, rb, lt, acc, a0, da, b0, db);
-      if constexpr (SPLIT) {  // the team's partial blocks: every lane of the team ends with the sum
+      if constexpr (SPLIT) {  // the team's partial blocks: its first lane ends with the sum
+        const int nw = ns < 32 ? ns : 32;  // lanes of the team in this warp
         const unsigned tmask =
-            ns == 32 ? 0xffffffffu : (((1u << ns) - 1u) << (threadIdx.x & 31u & ~(unsigned)(ns - 1)));
-        for (int o = ns >> 1; o > 0; o >>= 1) {
+            nw == 32 ? 0xffffffffu : (((1u << nw) - 1u) << (threadIdx.x & 31u & ~(unsigned)(nw - 1)));
+        for (int o = nw >> 1; o > 0; o >>= 1) {
 #pragma unroll
           for (int k = 0; k < TPT; ++k)
 #pragma unroll
             for (int f = 0; f < NFI; ++f) acc[k][f] += __shfl_xor_sync(tmask, acc[k][f], o);
+        }
+        if (ns > 32) {  // a block is one team: its four warps' sums
+          static_assert(SH::BLOCK == 128, "four warps");
+          __shared__ double s_part[3][S == 1 ? TPT * NFI : 1];
+          const int warp = (int)threadIdx.x >> 5;
+          __syncthreads();  // the previous quartet's sums are read
+          if (warp > 0 && (threadIdx.x & 31) == 0) {
+#pragma unroll
+            for (int k = 0; k < TPT; ++k)
+#pragma unroll
+              for (int f = 0; f < NFI; ++f) s_part[warp - 1][k * NFI + f] = acc[k][f];
+          }
+          __syncthreads();
+          if (threadIdx.x == 0) {
+#pragma unroll
+            for (int k = 0; k < TPT; ++k)
+#pragma unroll
+              for (int f = 0; f < NFI; ++f)
+                acc[k][f] += s_part[0][k * NFI + f] + s_part[1][k * NFI + f] + s_part[2][k * NFI + f];
+          }
         }
       }
     } else if constexpr (SLICE) {

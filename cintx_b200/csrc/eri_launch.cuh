@@ -38,8 +38,9 @@ __host__ __device__ constexpr bool class_valid(int li, int lj, int lk, int ll) {
 
 int device_sm_count();
 
-// Largest number of groups of s lanes that can share a quartet (0: the shape has no split form).
-__host__ __device__ constexpr int split_max(int s) { return s == 1 ? 32 : (s < 128 ? 128 / s : 0); }
+// Largest number of groups of s lanes that can share a quartet (0: the shape has no split form).  Teams
+// of one-lane groups are at most a warp, or a block of 128.
+__host__ __device__ constexpr int split_max(int s) { return s < 128 ? 128 / s : 0; }
 
 }  // namespace cintx
 #include "eri_splitcoop.cuh"
@@ -61,8 +62,9 @@ cudaError_t launch_eri(const LaunchArgs& a) {
     attr_done[dev] = 1;
   }
   if (a.nrec <= 0) return cudaSuccess;
-  // a team of nsplit groups must be a power of two inside one block (one warp for one-lane groups)
-  if (SPLIT && (a.nsplit < 1 || a.nsplit > split_max(SH::S) || (a.nsplit & (a.nsplit - 1)) != 0))
+  // a team of nsplit groups must be a power of two inside one block (for one-lane groups not two warps)
+  if (SPLIT && (a.nsplit < 1 || a.nsplit > split_max(SH::S) || (a.nsplit & (a.nsplit - 1)) != 0 ||
+                (SH::S == 1 && a.nsplit == 64)))
     return cudaErrorInvalidValue;
   const int per_block = SPLIT ? SH::Q / a.nsplit : SH::Q;
   long long blocks = ((long long)a.nrec + per_block - 1) / per_block;
