@@ -159,7 +159,10 @@ struct EriShape {
   static constexpr bool ROLL_ROOTS = SLICE && (S >= 8 || ROLL);
   // resident blocks requested from the register allocator: <= 128 registers per thread for the
   // multi-lane kernels (their stalls are latency bound and need warps)
-  static constexpr int MINB = S == 1 ? 1 : (65536 / (BLOCK * REGS) > 0 ? 65536 / (BLOCK * REGS) : 1);
+  // one-lane classes of at most 10 functions fit 128 registers without a spill, four blocks in place of
+  // three ((10|10) 148 registers uncapped, (11|00) 142, (30|00) 138, (20|00) 130: 4 to 9% faster over a
+  // 120-atom molecule); at 18 functions the cap spills and costs (20|10) up to 10%
+  static constexpr int MINB = S == 1 ? (NFI * NTUP <= 10 ? 4 : 1) : (65536 / (BLOCK * REGS) > 0 ? 65536 / (BLOCK * REGS) : 1);
   static constexpr int Q = BLOCK / LANES;
   // one-lane classes of low order stage their root-table block in shared memory: the lanes'
   // scattered coefficient loads then cost shared-memory wavefronts instead of L1 sectors
