@@ -1,5 +1,6 @@
-"""Quartets whose primitive quartets are shared by several lane groups (prim_split): single-block
-calls and short lists of contracted shells, where the split is widest, against the CPU oracle."""
+"""The edges of the launch rules: quartets whose primitive quartets are shared by several lane groups
+(prim_split; single-block calls and short lists of contracted shells, where the split is widest), roots at
+the end of the table, and J/K contractions of every ket size, against the CPU oracle or the plain path."""
 import numpy as np
 import pytest
 
@@ -77,3 +78,54 @@ def test_derivatives_of_contracted_shells(nsh, sph):
             one, _ = f(t[q], mol.atm, mol.bas, mol.env, opt=opt)
             # equal up to the order of at most 169 x 169 primitive terms of either sign
             assert np.allclose(one, got[off[q]:off[q] + one.size], rtol=1e-9, atol=1e-11)
+
+
+@pytest.mark.parametrize("ls", [(0, 0, 0, 0), (1, 0, 1, 0), (2, 0, 2, 0), (2, 1, 2, 1), (2, 2, 2, 2), (3, 2, 3, 2)])
+def test_roots_at_the_end_of_the_table(ls):
+    """Quartets whose x lies on, just below and just above the last table interval of their order and
+    the 2^-20 before it where the large-x form starts (xmax of rys_roots, per order 1..6)."""
+    import cintx_b200 as cx
+    from oracle import Restatement
+    n = sum(ls) // 2 + 1
+    xmax = {1: 40, 2: 52, 3: 60, 4: 64, 5: 72, 6: 76}[n]
+    orc = Restatement()
+    for eps in (-1e-3, -2.0 ** -20 / xmax, -1e-9, 0.0, 1e-15, 1e-9, 1e-3):
+        a = 0.7  # four equal exponents: a_ij = a_kl = 2a, rho = a, x = a R^2
+        r = float(np.sqrt(xmax * (1.0 + eps) / a))
+        mol = M.build_molecule("ends", [[0.0, 0.0, 0.0], [0.6 * r, 0.48 * r, 0.64 * r]],
+                               [[M.ShellSpec(l, [a], [1.0]) for l in ls[:2]], [M.ShellSpec(l, [a], [1.0]) for l in ls[2:]]])
+        q = np.array([[0, 1, 2, 3]], dtype=np.int32)
+        ref, _ = orc.int2e_batch(q, mol, sph=True)
+        got, _ = cx.int2e_sph(q[0], mol.atm, mol.bas, mol.env)
+        assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max() + 1e-15, (ls, eps)
+
+
+@pytest.mark.parametrize("sph", [True, False])
+def test_jk_of_shells_up_to_g(sph):
+    """J and K over every ket extent the contraction has a kernel for (spherical 1..9; cartesian up to
+    10, and 15 in the general kernel) against einsum over the sweep's own s1 tensor."""
+    import cintx_b200 as cx
+    import torch
+    mol = contracted([0, 1, 2, 3, 4], [2, 1, 1, 1, 1], 13)
+    l = mol.bas[:, 1].astype(int)
+    nao = int((2 * l + 1 if sph else (l + 1) * (l + 2) // 2).sum())
+    g = torch.Generator(device="cuda").manual_seed(3)
+    dm = torch.randn(nao, nao, generator=g, device="cuda", dtype=torch.float64)
+    dm = dm + dm.T
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+        plan = cx.Plan.screened(opt, 1e-14, sph=sph)
+        eri = torch.full((nao ** 4,), np.nan, dtype=torch.float64, device="cuda")
+        s = torch.cuda.current_stream().cuda_stream
+        plan.execute_ao(eri.data_ptr(), eri.numel(), 1, s)
+        vj, vk, j2, k2 = (torch.empty(nao, nao, dtype=torch.float64, device="cuda") for _ in range(4))
+        plan.jk(dm.data_ptr(), nao, vj.data_ptr(), vk.data_ptr(), s)
+        plan.jk(dm.data_ptr(), nao, j2.data_ptr(), 0, s)
+        plan.jk(dm.data_ptr(), nao, 0, k2.data_ptr(), s)
+        torch.cuda.synchronize()
+        plan.close()
+    eri = eri.reshape(nao, nao, nao, nao)
+    assert torch.isfinite(eri).all()
+    for got, ref in ((vj, torch.einsum("pqrs,rs->pq", eri, dm)), (vk, torch.einsum("pqrs,qs->pr", eri, dm))):
+        # nao^2 products a sum; eps times their absolute sum bounds a difference in the order of addition
+        assert (got - ref).abs().max() <= 1e-15 * nao ** 2 * float(eri.abs().max() * dm.abs().max())
+    assert (j2 - vj).abs().max() <= 1e-11 * vj.abs().max() and (k2 - vk).abs().max() <= 1e-11 * vk.abs().max()
