@@ -103,6 +103,12 @@ struct Segment {
   long long nout = 0;      // doubles per block (screened)
   long long out_off = 0;   // chunk-relative output start of this segment
   double flops = 0;        // algorithmic FP64 flops of the segment
+  double work = 0;         // its primitive quartets
+  // relative run time, for spreading a sweep over graph branches: finding a primitive quartet's roots and
+  // prefactor costs about as much as 120 of its flops ((00|00) 13 ps per primitive quartet and 18 flops,
+  // (10|10) 25 ps and 174), and a launch some microseconds (tuned 40-atom sweep 4.98 -> 4.85 ms against
+  // branches balanced by flops)
+  double cost() const { return flops + 120.0 * work + 3e7; }
   int range0 = 0;          // merged class segments (tile == -2): GenRange slice
   int nranges = 0;
   bool fp32 = false;       // FP32 recurrences (mixed-precision plans)
@@ -537,6 +543,7 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
     Segment& sg = ch.segs[i];
     const PrimSplit ps = prim_split(sg.li, sg.lj, sg.lk, sg.ll, seg_work[i].first, sg.nrec, seg_work[i].second);
     sg.nsplit = ps.ns;
+    sg.work = seg_work[i].first;
     if (ps.ns > 1 && ps.pmin > 0) heavy.emplace_back(i, ps.pmin);
   }
   {
@@ -575,6 +582,8 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
     rest.flops = big.flops * ws / (wb + ws);
     big.nrec = mid - r0;
     big.flops -= rest.flops;
+    big.work = wb;
+    rest.work = ws;
     ch.segs.insert(ch.segs.begin() + heavy[h].first + 1, rest);
   }
   ch.out_size = off;
@@ -1518,11 +1527,11 @@ int cintx_plan_graph_build(CintxPlan* p, const int64_t* chunks, int64_t n, doubl
     // longest-first assignment of class segments to branches
     std::vector<int> idx(ch.segs.size());
     std::iota(idx.begin(), idx.end(), 0);
-    std::sort(idx.begin(), idx.end(), [&](int a, int b) { return ch.segs[a].flops > ch.segs[b].flops; });
+    std::sort(idx.begin(), idx.end(), [&](int a, int b) { return ch.segs[a].cost() > ch.segs[b].cost(); });
     std::vector<double> load(nbranch, 0.0);
     for (int i : idx) {
       const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-      load[b] += ch.segs[i].flops + 1.0;
+      load[b] += ch.segs[i].cost();
       if (rc || (rc = run_segment(p, ch.segs[i], out_dev, p->branches[b], ds, ts, false))) {
         cudaGraph_t g;
         cudaStreamEndCapture(origin, &g);
@@ -2105,6 +2114,12 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
     }
     ch.segs.clear();
     long long rec = 0;
+    // mean primitive quartets of a piece's quartets (a tile's pairs have counts within a half octave
+    // each, or for 3-centre tiles up to their shells' products)
+    auto piece_np = [&](int i) {
+      const Tile& t = p->tiles[ch.pieces[i].tile];
+      return (double)t.nprimq / (double)t.row_prefix.back();
+    };
     // one class's pieces, all in one segment, or its large quartets (prim_split) in one and the rest in another
     auto add_segment = [&](const std::vector<int>& mem, int nsplit) {
       const Segment& p0 = ch.pieces[mem[0]];
@@ -2142,16 +2157,11 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
         p->ranges.push_back(g);
         m.nrec += pc.t1 - pc.t0;
         m.flops += pc.flops;
+        m.work += (double)(pc.t1 - pc.t0) * piece_np(i);
       }
       m.nranges = (int)p->ranges.size() - m.range0;
       rec += m.nrec;
       ch.segs.push_back(m);
-    };
-    // mean primitive quartets of a piece's quartets (a tile's pairs have counts within a half octave
-    // each, or for 3-centre tiles up to their shells' products)
-    auto piece_np = [&](int i) {
-      const Tile& t = p->tiles[ch.pieces[i].tile];
-      return (double)t.nprimq / (double)t.row_prefix.back();
     };
     for (auto& mem : members) {
       const Segment& p0 = ch.pieces[mem[0]];
