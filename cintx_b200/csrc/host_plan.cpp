@@ -104,10 +104,10 @@ struct Segment {
   long long out_off = 0;   // chunk-relative output start of this segment
   double flops = 0;        // algorithmic FP64 flops of the segment
   double work = 0;         // its primitive quartets
-  // relative run time, for spreading a sweep over graph branches: finding a primitive quartet's roots and
-  // prefactor costs about as much as 120 of its flops ((00|00) 13 ps per primitive quartet and 18 flops,
-  // (10|10) 25 ps and 174), and a launch some microseconds (tuned 40-atom sweep 4.98 -> 4.85 ms against
-  // branches balanced by flops)
+  // relative run time, for spreading segments over streams and graph branches: finding a primitive
+  // quartet's roots and prefactor costs about as much as 120 of its flops ((00|00) 13 ps per primitive
+  // quartet and 18 flops, (10|10) 25 ps and 174), and a launch some microseconds (against balancing by
+  // flops: tuned 40-atom sweep 4.98 -> 4.85 ms, cartesian 19-atom sweep 1082 -> 1036 us)
   double cost() const { return flops + 120.0 * work + 3e7; }
   int range0 = 0;          // merged class segments (tile == -2): GenRange slice
   int nranges = 0;
@@ -704,13 +704,12 @@ static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_
   }
   std::vector<int> idx(n);
   std::iota(idx.begin(), idx.end(), 0);
-  std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return ch.segs[a].flops > ch.segs[b].flops; });
+  std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return ch.segs[a].cost() > ch.segs[b].cost(); });
   Fork fork(stream, side, n - 1);
   for (int i : idx) {
     const Segment& sg = ch.segs[i];
-    // a launch costs some microseconds however small its work
     cudaStream_t st =
-        fork.next(sg.flops + 3e7, class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant));
+        fork.next(sg.cost(), class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant));
     if (fork.error() != cudaSuccess) break;
     if ((rc = run_segment(p, sg, out_dev, st, ds, ts, false)) || (after && (rc = after(sg, st)))) break;
   }
