@@ -102,6 +102,9 @@ int default_variant(int li, int lj, int lk, int ll) {
   if (lanes(7) > 0) return 7;
   for (int v : {11, 10})
     if (splitcoop_applies(li, lj, lk, ll, v)) return v;
+  // 256 lanes with more accumulators than 128 registers hold: 255 registers
+  const int s = default_threads(li, lj, lk, ll), ntup = ncart(lj) * ncart(lk) * ncart(ll);
+  if ((ntup + s - 1) / s * ncart(li) > 40) return 1;
   return 0;
 }
 

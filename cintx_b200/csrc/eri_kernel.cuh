@@ -70,9 +70,9 @@ __host__ __device__ constexpr int default_threads(int li, int lj, int lk, int ll
 }
 
 // Launch-shape variants the autotuner chooses between: the accumulator budget per lane and the
-// register cap of multi-lane shapes (variant 0 is the default shape, used by plans that are not
-// autotuned).  A 255-register cap halves the resident blocks but removes the spills that the
-// 128-register cap forces on most d/f/g multi-lane classes.
+// register cap of multi-lane shapes (variant 0 is the default shape; plans that are not autotuned start
+// with the variant that default_variant gives).  A 255-register cap halves the resident blocks but
+// removes the spills that the 128-register cap forces on most d/f/g multi-lane classes.
 // Variants 4, 5 and 6 ("sliced") run a multi-lane class without any barrier inside the primitive
 // loop: every lane evaluates the roots and all 3*NR recurrences itself in registers and
 // accumulates its own slice of (j,k,l) tuples (redundant FP64 work for no shared-memory

@@ -255,6 +255,7 @@ constexpr int kLaunchVariants = 12;
 //                                recurrences in registers, no barrier per primitive quartet;
 //   up to 4 lanes of 48          the same with the roots rolled (7), tables of at most 72 doubles;
 //   64 lanes or more             split horizontal transfers (11: 24 accumulators per lane, else 10: 12);
+//   over 40 accumulators a lane  (256 lanes, several g shells) the default shape with 255 registers (1);
 //   the rest                     the default shape.
 // All classes of a 120-atom s/p/d/f molecule, one after another: default shapes 274.7 ms, this rule
 // 202.6, the fastest shape of each class as timed by the autotuner 202.1; 3-centre sweep of 40 atoms 3.84,

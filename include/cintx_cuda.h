@@ -312,8 +312,9 @@ CINTX_API int cintx_tuned_shapes_export(int *records, int cap);
 CINTX_API int cintx_tuned_shapes_import(const int *records, int n);
 /* Sets the launch-shape variant (0..11) of every segment, for tests and tuning scripts; a class
  * that the variant does not apply to runs its default shape.  (A new plan's segments start with the
- * variant a rule on the class's size gives, which is the default shape 0 for some classes only.)  Returns the number of segments
- * changed (or -1).  A graph captured earlier is released when anything changed. */
+ * variant that a rule on the class's size gives, which is the default shape 0 for some classes only.)
+ * Returns the number of segments changed (or -1).  A graph captured earlier is released when anything
+ * changed. */
 CINTX_API int cintx_plan_set_shape(CintxPlan *plan, int variant);
 /* Lanes per quartet of each segment of a chunk (as chosen by the autotuner, or the default
  * shape).  Returns the segment count (or -1). */
