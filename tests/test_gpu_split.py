@@ -129,3 +129,54 @@ def test_jk_of_shells_up_to_g(sph):
         # nao^2 products a sum; eps times their absolute sum bounds a difference in the order of addition
         assert (got - ref).abs().max() <= 1e-15 * nao ** 2 * float(eri.abs().max() * dm.abs().max())
     assert (j2 - vj).abs().max() <= 1e-11 * vj.abs().max() and (k2 - vk).abs().max() <= 1e-11 * vk.abs().max()
+
+
+def test_forked_execution_from_two_threads_and_under_capture():
+    """One explicit plan run by two host threads on streams of their own, and captured into a graph by
+    the caller (where it stays on the captured stream), gives what a single run gives."""
+    import threading
+
+    import cintx_b200 as cx
+    import torch
+    mol = contracted([0, 0, 1, 1, 2], [8, 1, 3, 1, 1], 15)
+    i, j = np.tril_indices(mol.nbas)
+    a, b = np.tril_indices(i.size)
+    q = np.stack([i[a], j[a], i[b], j[b]], axis=1).astype(np.int32)
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+        plan = cx.Plan.shells(opt, cx.INT2E, q)
+        n = plan.stats.nintegrals
+        ref = torch.zeros(n, dtype=torch.float64, device="cuda")
+        plan.execute(ref.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        bad, outs = [], [torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(2)]
+
+        def work(k):
+            try:
+                s = torch.cuda.Stream()
+                with torch.cuda.stream(s):
+                    for _ in range(20):
+                        outs[k].zero_()
+                        plan.execute(outs[k].data_ptr(), stream=s.cuda_stream)
+                        got = outs[k].clone()
+                        s.synchronize()
+                        if not torch.equal(got, ref):
+                            bad.append(k)
+            except Exception as e:  # noqa: BLE001
+                bad.append(e)
+
+        th = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+        for t in th:
+            t.start()
+        for t in th:
+            t.join()
+        assert not bad
+        out = torch.zeros(n, dtype=torch.float64, device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            plan.execute(out.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+        del graph
+        plan.close()
