@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "common.h"
 
@@ -648,17 +649,34 @@ cudaError_t launch_block_absmax_sqrt(const QuartetRec* recs, long long nrec, con
   return cudaGetLastError();
 }
 
+// Most dynamic shared memory of a jk_contract_group_kernel block (of the 227 KB a block may have).
+constexpr size_t kJkSmem = 200 * 1024;
+
+static int jk_group_lanes(int nij) {
+  int G = 1;
+  while (G < 32 && G < nij) G *= 2;
+  return G;
+}
+static size_t jk_group_smem(int nij, int nk, int nl) {
+  return sizeof(double) * (size_t)jk_group_doubles(nij, nk, nl) * (32 * kJkWarps / jk_group_lanes(nij));
+}
+
 template <int NK, int NL>
 static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
                                    const double* dm, int nao, double* A, double* B,
                                    cudaStream_t stream, int ni, int nj) {
-  int G = 1;
-  while (G < 32 && G < ni * nj) G *= 2;
-  const size_t smem = sizeof(double) * (size_t)jk_group_doubles(ni * nj, NK, NL) * (32 * kJkWarps / G);
+  const int G = jk_group_lanes(ni * nj);
+  const size_t smem = jk_group_smem(ni * nj, NK, NL);
   auto kern = jk_contract_group_kernel<NK, NL>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // The limit is a property of the kernel that all host threads share, and one instance serves bras of
+  // several sizes: it is set to what the largest may take, never to this launch's own size.
+  static std::atomic<int> attr_done[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !attr_done[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJkSmem);
     if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) attr_done[dev] = 1;
   }
   const long long resident = 148LL * 16 * (32 / G);  // groups, 16 warps per SM
   const int run = (int)std::max(1LL, std::min<long long>(kJkRun, nrec / (2 * resident)));
@@ -693,7 +711,7 @@ cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int
 #undef CINTX_JK_THREAD
 #define CINTX_JK(K, L) \
   if (nk == K && nl == L) return launch_jk_group<K, L>(recs, nrec, pao, out, dm, nao, A, B, stream, ni, nj);
-  if (jk_group_doubles(ni * nj, nk, nl) * sizeof(double) * kJkWarps <= 200 * 1024) {
+  if (jk_group_smem(ni * nj, nk, nl) <= kJkSmem) {
     CINTX_JK(1, 1) CINTX_JK(3, 1) CINTX_JK(3, 3)  // (1, 1) and (3, 1): cartesian g first shells
     CINTX_JK(5, 1) CINTX_JK(5, 3) CINTX_JK(5, 5)
     CINTX_JK(6, 1) CINTX_JK(6, 3) CINTX_JK(6, 6)

@@ -180,3 +180,46 @@ def test_forked_execution_from_two_threads_and_under_capture():
         assert torch.equal(out, ref)
         del graph
         plan.close()
+
+
+@pytest.mark.parametrize("sph", [True, False])
+def test_jk_from_two_threads(sph):
+    """Two host threads build J and K on plans of their own, streams of their own.  The kets of the f and
+    g shells take shared memory that differs from bra to bra under one kernel ((gf|gf) and (gg|gf), or
+    cartesian (fd|fd) and (ff|fd)), so a launch that set the kernel's limit to its own size would have
+    the other thread's larger one refused."""
+    import threading
+
+    import cintx_b200 as cx
+    import torch
+    mol = contracted([3, 4] if sph else [0, 2, 3], [1, 1, 1], 17)
+    l = mol.bas[:, 1].astype(int)
+    nao = int((2 * l + 1 if sph else (l + 1) * (l + 2) // 2).sum())
+    g = torch.Generator(device="cuda").manual_seed(5)
+    dm = torch.randn(nao, nao, generator=g, device="cuda", dtype=torch.float64)
+    dm = dm + dm.T
+    torch.cuda.synchronize()
+    bad, res = [], [None, None]
+
+    def work(k):
+        try:
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s), cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+                plan = cx.Plan.screened(opt, 1e-14, sph=sph)
+                vj, vk = (torch.empty(nao, nao, dtype=torch.float64, device="cuda") for _ in range(2))
+                for _ in range(300):
+                    plan.jk(dm.data_ptr(), nao, vj.data_ptr(), vk.data_ptr(), s.cuda_stream)
+                s.synchronize()
+                res[k] = (vj, vk)
+                plan.close()
+        except Exception as e:  # noqa: BLE001
+            bad.append(e)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not bad, bad
+    for a, b in zip(*res):  # the atomic adds of a sum come in any order
+        assert (a - b).abs().max() <= 1e-12 * a.abs().max()
