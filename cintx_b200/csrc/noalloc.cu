@@ -187,7 +187,9 @@ extern "C" int cintx_int2e_noalloc(double* out_dev, const int* shls, int64_t n, 
               src[0] = p2[0]; src[1] = p2[1]; src[2] = p1[0]; src[3] = p1[1];
             }
             GKey k{l[src[0]], l[src[1]], l[src[2]], l[src[3]], ast[src[0]], ast[src[1]], ast[src[2]], ast[src[3]]};
-            if (class_needs_scratch(k.li, k.lj, k.lk, k.ll, sp)) {
+            // a property of the class: asked once per group, not per quartet (lists of 4000 quartets: 436 -> 354 us)
+            const auto group = groups.try_emplace(k);
+            if (group.second && class_needs_scratch(k.li, k.lj, k.lk, k.ll, sp)) {
               set_error(CINTX_STATUS_UNSUPPORTED_API,
                         "this entry point does not evaluate classes with two or more g shells; use the plan API");
               return CINTX_STATUS_UNSUPPORTED_API;
@@ -197,7 +199,7 @@ extern "C" int cintx_int2e_noalloc(double* out_dev, const int* shls, int64_t n, 
             r.pkl = swap ? id1 : id2;
             r.out = off;
             for (int a = 0; a < 4; ++a) r.out += (long long)cs[a] * ne[a] * ast[a];
-            groups[k].push_back(r);
+            group.first->second.push_back(r);
           }
     off += st;
   }
