@@ -480,7 +480,7 @@ class Plan:
         return n
 
     def set_shape(self, variant: int) -> int:
-        """Runs every segment in launch-shape variant `variant` (0 = default shape)."""
+        """Runs every quartet on one group of lanes in launch-shape variant `variant` (0 = default shape)."""
         n = lib.cintx_plan_set_shape(self.handle, variant)
         if n < 0:
             _check(last_error()[0])

@@ -114,7 +114,10 @@ struct Segment {
   bool fp32 = false;       // FP32 recurrences (mixed-precision plans)
   double prim_eps = 0;     // primitive Schwarz threshold (tuned plans)
   int variant = 0;         // launch shape: default_variant, or the choice of cintx_plan_autotune
-  int nsplit = 1;          // groups sharing each quartet's primitive quartets (prim_split); > 1: default shape
+  int nsplit = 1;          // groups sharing each quartet's primitive quartets by prim_split's rule
+  bool forced = false;     // cintx_plan_set_shape: every quartet whole, in shape `variant`
+  // groups per quartet of a launch; more than one run the default shape's split form, whatever `variant` is
+  int groups() const { return forced ? 1 : nsplit; }
   bool swap = false;       // screened: the tile's records are (col, row) pairs
 };
 
@@ -624,6 +627,11 @@ static int gen_records(CintxPlan* p, const Segment* s0, const Segment* s1, cudaS
   return CINTX_STATUS_SUCCESS;
 }
 
+// Whether a segment's launch keeps its transform buffers in device scratch (split launches never do).
+static bool segment_scratch(const CintxPlan* p, const Segment& sg) {
+  return sg.groups() == 1 && class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant);
+}
+
 // Runs one segment's class kernel; gen: its records are written first (else they are there already).
 static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStream_t stream, DeviceState* ds,
                        ThreadScratch* ts, bool gen) {
@@ -660,7 +668,7 @@ static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStr
     cudaError_t e = launch_class(sg.li, sg.lj, sg.lk, sg.ll, p->sph, recs + r0, nr, o->d_pairs, o->d_prims,
                                  out_dev + sg.out_off, sg.strides >= 0 ? p->stride_sets[sg.strides] : one_stride(sg.st), sg.expcutoff, ds->rys, stream, sg.fp32, sg.prim_eps,
                                  sg.variant, rb ? p->d_rootbuf : nullptr, rb ? p->d_rootbase + sg.rec0 + r0 : nullptr,
-                                 sg.nsplit);
+                                 sg.groups());
     if (e != cudaSuccess) {
       set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("kernel launch failed: ") + cudaGetErrorString(e));
       return CINTX_STATUS_EXECUTION_FAILED;
@@ -708,8 +716,7 @@ static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_
   Fork fork(stream, side, n - 1);
   for (int i : idx) {
     const Segment& sg = ch.segs[i];
-    cudaStream_t st =
-        fork.next(sg.cost(), class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant));
+    cudaStream_t st = fork.next(sg.cost(), segment_scratch(p, sg));
     if (fork.error() != cudaSuccess) break;
     if ((rc = run_segment(p, sg, out_dev, st, ds, ts, false)) || (after && (rc = after(sg, st)))) break;
   }
@@ -1359,7 +1366,10 @@ int cintx_plan_autotune(CintxPlan* p, int64_t chunk, double* out_dev, void* stre
   for (Chunk& ch : p->chunks)
     for (Segment& sg : ch.segs) {
       auto it = best.find(std::make_tuple(sg.li, sg.lj, sg.lk, sg.ll, (int)sg.fp32));
-      if (it != best.end()) sg.variant = it->second;
+      if (it != best.end()) {
+        sg.variant = it->second;
+        sg.forced = false;
+      }
     }
   if (p->gexec) {  // the captured graph holds the old launch shapes
     cudaGraphExecDestroy(p->gexec);
@@ -1383,6 +1393,7 @@ int cintx_plan_use_tuned_shapes(CintxPlan* p) {
       auto it = g_tuned.find(std::make_tuple(dev, sg.li, sg.lj, sg.lk, sg.ll, (int)sg.fp32));
       if (it != g_tuned.end()) {
         sg.variant = it->second;
+        sg.forced = false;
         ++applied;
       }
     }
@@ -1451,8 +1462,9 @@ int cintx_plan_set_shape(CintxPlan* p, int variant) {
   int changed = 0;
   for (Chunk& ch : p->chunks)
     for (Segment& sg : ch.segs) {
-      changed += sg.variant != variant;
+      changed += sg.variant != variant || sg.groups() != 1;
       sg.variant = variant;
+      sg.forced = true;
     }
   if (changed && p->gexec) {
     cudaGraphExecDestroy(p->gexec);
@@ -1464,8 +1476,10 @@ int cintx_plan_set_shape(CintxPlan* p, int variant) {
 int cintx_plan_segment_lanes(const CintxPlan* p, int64_t chunk, int* lanes, int cap) {
   if (!p || chunk < 0 || chunk >= (int64_t)p->chunks.size()) return -1;
   const std::vector<Segment>& segs = p->chunks[chunk].segs;
-  for (int i = 0; i < (int)segs.size() && i < cap && lanes; ++i)
-    lanes[i] = variant_lanes(segs[i].li, segs[i].lj, segs[i].lk, segs[i].ll, p->sph, segs[i].fp32, segs[i].variant);
+  for (int i = 0; i < (int)segs.size() && i < cap && lanes; ++i) {
+    const int v = segs[i].groups() > 1 ? 0 : segs[i].variant;
+    lanes[i] = segs[i].groups() * variant_lanes(segs[i].li, segs[i].lj, segs[i].lk, segs[i].ll, p->sph, segs[i].fp32, v);
+  }
   return (int)segs.size();
 }
 
@@ -1485,7 +1499,7 @@ int cintx_plan_graph_build(CintxPlan* p, const int64_t* chunks, int64_t n, doubl
       return CINTX_STATUS_INVALID_INPUT;
     }
     for (const Segment& sg : p->chunks[c].segs)
-      if (class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant)) {
+      if (segment_scratch(p, sg)) {
         set_error(CINTX_STATUS_UNSUPPORTED_API, "plan contains classes with device scratch; use cintx_plan_execute");
         return CINTX_STATUS_UNSUPPORTED_API;
       }

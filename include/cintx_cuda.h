@@ -312,12 +312,14 @@ CINTX_API int cintx_tuned_shapes_export(int *records, int cap);
 CINTX_API int cintx_tuned_shapes_import(const int *records, int n);
 /* Sets the launch-shape variant (0..11) of every segment, for tests and tuning scripts; a class
  * that the variant does not apply to runs its default shape.  (A new plan's segments start with the
- * variant that a rule on the class's size gives, which is the default shape 0 for some classes only.)
- * Returns the number of segments changed (or -1).  A graph captured earlier is released when anything
- * changed. */
+ * variant that a rule on the class's size gives, which is the default shape 0 for some classes only,
+ * and those of heavily contracted quartets share each quartet over several groups of the default
+ * shape's lanes; here every quartet runs on one group of the shape asked for, until tuned shapes are
+ * applied.)  Returns the number of segments changed (or -1).  A graph captured earlier is released
+ * when anything changed. */
 CINTX_API int cintx_plan_set_shape(CintxPlan *plan, int variant);
-/* Lanes per quartet of each segment of a chunk (as chosen by the autotuner, or the default
- * shape).  Returns the segment count (or -1). */
+/* Lanes per quartet of each segment of a chunk, of all groups that share a quartet together, in the
+ * shape the segment runs in.  Returns the segment count (or -1). */
 CINTX_API int cintx_plan_segment_lanes(const CintxPlan *plan, int64_t chunk, int *lanes, int cap);
 /* End to end: evaluates one chunk (chunk >= 0) or every chunk (chunk < 0) into device staging
  * buffers and copies the output to host memory out_host, chunks back to back (out_host holds the

@@ -223,3 +223,34 @@ def test_jk_from_two_threads(sph):
     assert not bad, bad
     for a, b in zip(*res):  # the atomic adds of a sum come in any order
         assert (a - b).abs().max() <= 1e-12 * a.abs().max()
+
+
+@pytest.mark.parametrize("ls", [(2, 1, 1, 1), (2, 0, 2, 0), (3, 2, 2, 1)])
+def test_set_shape_runs_the_shape_on_split_quartets(ls):
+    """Two contracted quartets, which a plan of their own shares over lane groups, and the same two
+    repeated 6000 times, which no rule splits: in each forced shape both plans run the same kernel on one
+    group per quartet, so their blocks agree to the last bit, and both report the shape's lanes."""
+    import cintx_b200 as cx
+    import torch
+    mol = contracted(list(ls), [3, 3, 3, 3], 21)
+    q = np.array([[0, 5, 10, 3], [4, 9, 2, 7]], dtype=np.int32)
+    s = torch.cuda.current_stream().cuda_stream
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+        few, many = cx.Plan.shells(opt, cx.INT2E, q), cx.Plan.shells(opt, cx.INT2E, np.tile(q, (6000, 1)))
+        n = few.stats.nintegrals
+        a = torch.empty(n, dtype=torch.float64, device="cuda")
+        b = torch.empty(many.stats.nintegrals, dtype=torch.float64, device="cuda")
+        split_lanes = few.segment_lanes(0)
+        few.execute(a.data_ptr(), stream=s)
+        split = a.clone()
+        for v in range(12):
+            few.set_shape(v), many.set_shape(v)
+            assert few.set_shape(v) == 0  # nothing left to change
+            lanes = few.segment_lanes(0)
+            assert set(lanes) == set(many.segment_lanes(0)) and (v or (lanes < split_lanes).all())
+            few.execute(a.data_ptr(), stream=s)
+            many.execute(b.data_ptr(), stream=s)
+            assert torch.equal(a, b[:n]), v
+            # at most 81 terms of 1e-16 of the block's size each
+            assert (a - split).abs().max() <= 1e-13 * split.abs().max()
+        few.close(), many.close()
