@@ -473,7 +473,8 @@ class Plan:
                                          ctypes.c_void_p(stream)))
 
     def use_tuned_shapes(self) -> int:
-        """Reuse the launch shapes autotuned earlier in this process; returns segments changed."""
+        """Reuse the launch shapes autotuned earlier in this process; returns the number of segments
+        that have their tuned shape now."""
         n = lib.cintx_plan_use_tuned_shapes(self.handle)
         if n < 0:
             _check(1)

@@ -19,6 +19,7 @@
 #include <memory>
 #include <mutex>
 #include <numeric>
+#include <set>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -1272,9 +1273,12 @@ int cintx_plan_sample_quartets(const CintxPlan* p, uint64_t seed, int64_t n, int
 // and are spread over `nbranch` parallel branches by their flop estimate; chunks follow each
 // other because they share out_dev.
 // Launch shapes chosen by the autotuner, per device and class (li, lj, lk, ll, fp32): kept for
-// the life of the process so that later plans can reuse them (cintx_plan_use_tuned_shapes).
+// the life of the process so that later plans can reuse them (cintx_plan_use_tuned_shapes).  Only
+// classes that were timed are in it: a class whose segments are all split has one shape to run, which
+// says nothing about the shape for whole quartets that a larger molecule's plan needs.
 static std::mutex g_tuned_mu;
 static std::map<std::tuple<int, int, int, int, int, int>, int> g_tuned;
+static std::set<int> g_tuned_devices;  // where the autotuner ran or choices were loaded
 
 int cintx_plan_autotune(CintxPlan* p, int64_t chunk, double* out_dev, void* stream_, int reps) {
   clear_error();
@@ -1295,11 +1299,9 @@ int cintx_plan_autotune(CintxPlan* p, int64_t chunk, double* out_dev, void* stre
     for (int i = 0; i < (int)p->chunks[c].segs.size(); ++i) {
       const Segment& sg = p->chunks[c].segs[i];
       const auto key = std::make_tuple(sg.li, sg.lj, sg.lk, sg.ll, (int)sg.fp32);
+      if (sg.nsplit > 1) continue;  // runs the split form of the default shape: nothing to choose
       auto it = target.find(key);
-      const Segment* cur = it == target.end() ? nullptr : &p->chunks[it->second.first].segs[it->second.second];
-      // segments of split quartets run the default shape: timed only where a class has no other
-      if (!cur || (cur->nsplit > 1 && sg.nsplit == 1) ||
-          (chunk < 0 && (cur->nsplit > 1) == (sg.nsplit > 1) && cur->nrec < sg.nrec))
+      if (it == target.end() || (chunk < 0 && p->chunks[it->second.first].segs[it->second.second].nrec < sg.nrec))
         target[key] = std::make_pair(c, i);
     }
   cudaEvent_t e0, e1;
@@ -1321,7 +1323,7 @@ int cintx_plan_autotune(CintxPlan* p, int64_t chunk, double* out_dev, void* stre
     std::vector<int> lanes_seen;
     double best_ms = 1e300;
     int best_v = 0;
-    for (int v = 0; v < (sg0.nsplit > 1 ? 1 : kLaunchVariants) && !rc; ++v) {
+    for (int v = 0; v < kLaunchVariants && !rc; ++v) {
       const int shape = variant_shape(sg0.li, sg0.lj, sg0.lk, sg0.ll, p->sph, sg0.fp32, v);
       if (std::find(lanes_seen.begin(), lanes_seen.end(), shape) != lanes_seen.end()) continue;
       lanes_seen.push_back(shape);
@@ -1362,14 +1364,13 @@ int cintx_plan_autotune(CintxPlan* p, int64_t chunk, double* out_dev, void* stre
     for (const auto& kv : best)
       g_tuned[std::make_tuple(dev, std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first),
                               std::get<3>(kv.first), std::get<4>(kv.first))] = kv.second;
+    g_tuned_devices.insert(dev);
   }
-  for (Chunk& ch : p->chunks)
-    for (Segment& sg : ch.segs) {
+  for (int64_t c = 0; c < (int64_t)p->chunks.size(); ++c)
+    for (Segment& sg : p->chunks[c].segs) {
       auto it = best.find(std::make_tuple(sg.li, sg.lj, sg.lk, sg.ll, (int)sg.fp32));
-      if (it != best.end()) {
-        sg.variant = it->second;
-        sg.forced = false;
-      }
+      if (it != best.end()) sg.variant = it->second;
+      if (it != best.end() || (sg.nsplit > 1 && (chunk < 0 || c == chunk))) sg.forced = false;
     }
   if (p->gexec) {  // the captured graph holds the old launch shapes
     cudaGraphExecDestroy(p->gexec);
@@ -1388,11 +1389,13 @@ int cintx_plan_use_tuned_shapes(CintxPlan* p) {
   cudaGetDevice(&dev);
   int applied = 0;
   std::lock_guard<std::mutex> lk(g_tuned_mu);
+  const bool tuned = g_tuned_devices.count(dev) > 0;
   for (Chunk& ch : p->chunks)
     for (Segment& sg : ch.segs) {
       auto it = g_tuned.find(std::make_tuple(dev, sg.li, sg.lj, sg.lk, sg.ll, (int)sg.fp32));
-      if (it != g_tuned.end()) {
-        sg.variant = it->second;
+      if (it != g_tuned.end()) sg.variant = it->second;
+      // split segments have the one shape that the autotuner would leave them too
+      if (it != g_tuned.end() || (tuned && sg.nsplit > 1)) {
         sg.forced = false;
         ++applied;
       }
@@ -1446,6 +1449,7 @@ int cintx_tuned_shapes_import(const int* records, int n) {
     const int* r = records + 6 * i;
     g_tuned[std::make_tuple(dev, r[0], r[1], r[2], r[3], r[4] ? 1 : 0)] = r[5];
   }
+  if (n > 0) g_tuned_devices.insert(dev);
   return CINTX_STATUS_SUCCESS;
 }
 

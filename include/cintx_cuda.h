@@ -296,12 +296,15 @@ CINTX_API int cintx_plan_graph_launch(CintxPlan *plan, void *stream);
  * on the chunk where it has the most quartets; reps runs after one warm-up, CUDA events on
  * `stream`, output into out_dev of max_chunk_doubles) in each launch shape (lanes per quartet,
  * hence quartets per block) that gives a distinct shape, and keeps the fastest per class for
- * every chunk of the plan.  Synchronous.  A graph captured earlier is released: capture again
+ * every chunk of the plan.  Classes whose quartets all share lane groups (short lists of contracted
+ * shells) are not timed and leave no choice behind.  Synchronous.  A graph captured earlier is released: capture again
  * after tuning. */
 CINTX_API int cintx_plan_autotune(CintxPlan *plan, int64_t chunk, double *out_dev, void *stream, int reps);
 /* Applies the launch shapes the autotuner chose earlier in this process on the current device
- * (any plan) to this plan's matching classes; returns the number of segments changed (or -1).
- * A graph captured earlier is released when anything changed. */
+ * (any plan) to this plan's matching classes; returns the number of segments that have their tuned
+ * shape (or -1): those of a class that was timed and, once the autotuner has run or shapes were
+ * loaded, those whose quartets share lane groups, which have one shape to run.  A graph captured
+ * earlier is released when there are any. */
 CINTX_API int cintx_plan_use_tuned_shapes(CintxPlan *plan);
 /* The launch shapes the autotuner chose in this process on the current device, as records of six
  * ints (li, lj, lk, ll, fp32, variant): cintx_tuned_shapes_export writes up to cap records and

@@ -254,3 +254,30 @@ def test_set_shape_runs_the_shape_on_split_quartets(ls):
             # at most 81 terms of 1e-16 of the block's size each
             assert (a - split).abs().max() <= 1e-13 * split.abs().max()
         few.close(), many.close()
+
+
+def test_tuning_a_small_molecule_leaves_larger_ones_their_shapes():
+    """A plan whose quartets are all split has nothing to tune: it adds no choice for the process, counts
+    as tuned itself, and a larger plan that picks up the process's choices afterwards runs the shapes it
+    would have run before."""
+    import cintx_b200 as cx
+    import torch
+    mol = contracted([2, 1, 2, 1], [3, 3, 3, 3], 23)
+    q = np.array([[0, 5, 10, 3], [4, 9, 2, 7]], dtype=np.int32)
+    s = torch.cuda.current_stream().cuda_stream
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+        few, many = cx.Plan.shells(opt, cx.INT2E, q), cx.Plan.shells(opt, cx.INT2E, np.tile(q, (6000, 1)))
+        buf = torch.empty(many.stats.nintegrals, dtype=torch.float64, device="cuda")
+        many.use_tuned_shapes()  # of tests before this one
+        lanes, recs, split = many.segment_lanes(0), cx.tuned_shapes(), few.segment_lanes(0)
+        few.autotune(buf.data_ptr(), chunk=-1, stream=s, reps=1)
+        assert cx.tuned_shapes() == recs
+        assert few.use_tuned_shapes() == len(split) and np.array_equal(few.segment_lanes(0), split)
+        many.use_tuned_shapes()
+        assert np.array_equal(many.segment_lanes(0), lanes)
+        few.set_shape(4)
+        few.autotune(buf.data_ptr(), chunk=0, stream=s, reps=1)
+        assert np.array_equal(few.segment_lanes(0), split)  # tuning ends a forced shape
+        many.autotune(buf.data_ptr(), chunk=-1, stream=s, reps=1)
+        assert many.use_tuned_shapes() == len(lanes) and len(cx.tuned_shapes()) >= 1
+        few.close(), many.close()
