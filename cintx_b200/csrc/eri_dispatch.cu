@@ -9,7 +9,8 @@ namespace cintx {
 cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const QuartetRec* recs, int nrec,
                          const ShellPair* pairs, const PrimPair* prims, double* out, const StrideSet& st,
                          double expcutoff, const RysTable& rys, cudaStream_t stream, bool fp32,
-                         double prim_eps, int variant, const double* rootbuf, const long long* rootbase, int nsplit) {
+                         double prim_eps, int variant, const double* rootbuf, const long long* rootbase, int nsplit,
+                         int chain) {
   LaunchArgs a;
   a.recs = recs;
   a.nrec = nrec;
@@ -27,6 +28,7 @@ cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const Quartet
   a.rootbuf = rootbuf;
   a.rootbase = rootbase;
   a.nsplit = nsplit;
+  a.chain = chain;
   return dispatch_eri(li, lj, lk, ll, sph, a);
 }
 

@@ -20,7 +20,7 @@
 // oriented like the plain kernel's.
 //
 // All derivatives of a 4-atom s/p/d/f molecule (84 000 tuples): 140.8 ms of device time with one pass per
-// component, one group per quartet and one launch after another; 3.9 ms so, launches forked.
+// component, one group per quartet and one launch after another; 3.9 ms so, launches overlapping (chain.cuh).
 #pragma once
 #include "eri_launch.cuh"
 
@@ -128,7 +128,9 @@ template <int LI, int LJ, int LK, int LL, bool SPH>
 __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
     eri_ip1_kernel(const QuartetRec* __restrict__ recs, int nrec, const ShellPair* __restrict__ pairs,
                    const PrimPair* __restrict__ prims, double* __restrict__ out,
-                   const __grid_constant__ StrideSet sts, long long scomp, double expcutoff, const __grid_constant__ RysTable rys, int nsplit) {
+                   const __grid_constant__ StrideSet sts, long long scomp, double expcutoff, const __grid_constant__ RysTable rys, int nsplit,
+                   int chain, int nblocks) {
+  if (chain_begin(chain, nblocks)) return;
   using SH = Ip1Shape<LI, LJ, LK, LL, SPH>;
   static_assert(ip1_shape_violation<SH>() == 0, "an index of this ip1 launch shape can leave its buffer");
   constexpr int S = SH::S, NR = SH::NR, GSZ = SH::GSZ, NFI = SH::NFI, TPT = SH::TPT;
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(Ip1Shape<LI, LJ, LK, LL, SPH>::BLOCK, 1)
   const int ns = nsplit;  // groups sharing a quartet
   const int team = group / ns, sub = group % ns, per_block = SH::Q / ns;
   const int tl = sub * S + lane, tn = ns * S;  // lanes of a team
-  for (int q = (int)blockIdx.x * per_block + team; q < nrec; q += (int)gridDim.x * per_block) {
+  for (int q = (int)blockIdx.x * per_block + team; q < nrec; q += nblocks * per_block) {
     const QuartetRec rec = recs[q];
     const ShellPair pij = pairs[rec.pij];
     const ShellPair pkl = pairs[rec.pkl];
@@ -419,6 +421,7 @@ struct Ip1Args {
   RysTable rys;
   cudaStream_t stream;
   int nsplit;       // groups sharing a quartet (power of two)
+  int chain;        // kChainPrev, kChainNext (chain.cuh)
   int* shape;       // not null: launch nothing, write {lanes per group, most groups per quartet, groups per block}
 };
 
@@ -446,9 +449,8 @@ cudaError_t launch_ip1(const Ip1Args& a) {
   long long blocks = ((long long)a.nrec + per_block - 1) / per_block;
   const long long cap = (long long)device_sm_count() * 32;
   if (blocks > cap) blocks = cap;
-  kern<<<(unsigned)blocks, SH::BLOCK, SH::SMEM_BYTES, a.stream>>>(a.recs, a.nrec, a.pairs, a.prims, a.out, a.st,
-                                                                  a.scomp, a.expcutoff, a.rys, a.nsplit);
-  return cudaGetLastError();
+  return chain_launch(kern, (unsigned)blocks, SH::BLOCK, SH::SMEM_BYTES, a.stream, a.chain, a.recs, a.nrec, a.pairs,
+                      a.prims, a.out, a.st, a.scomp, a.expcutoff, a.rys, a.nsplit);
 }
 
 // Classes compiled for derivatives: the derivative pair (i, j) with li, lj <= 3 in either order,

@@ -20,6 +20,7 @@
 #include <type_traits>
 #include <utility>
 
+#include "chain.cuh"
 #include "common.h"
 #include "c2s_coef.h"
 #include "rys_roots.cuh"
@@ -607,7 +608,8 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
                  const PrimPair* __restrict__ prims, double* __restrict__ out,
                  const __grid_constant__ StrideSet sts, double expcutoff, const __grid_constant__ RysTable rys, double* __restrict__ gscratch,
                  double prim_eps, const double* __restrict__ rootbuf, const long long* __restrict__ rootbase,
-                 int nsplit) {
+                 int nsplit, int chain, int nblocks) {
+  if (chain_begin(chain, nblocks)) return;
   using SH = EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>;
   constexpr int S = SH::S, NR = SH::NR, GSZ = SH::GSZ, NFI = SH::NFI, TPT = SH::TPT;
   constexpr bool FP64 = std::is_same<R, double>::value;
@@ -655,7 +657,7 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
   const int team = SPLIT ? group / ns : group, sub = SPLIT ? group % ns : 0;
   const int per_block = SPLIT ? SH::Q / ns : SH::Q;  // quartets a block holds
   const int qfirst = SLICE ? (int)blockIdx.x * SH::Q + (group & ~31) : (int)blockIdx.x * per_block + team;
-  for (int qb = qfirst; qb < nrec; qb += gridDim.x * per_block) {
+  for (int qb = qfirst; qb < nrec; qb += nblocks * per_block) {
     const int qv = SLICE ? qb + (group & 31) : qb;
     const bool live = !SLICE || qv < nrec;
     const int q = live ? qv : nrec - 1;

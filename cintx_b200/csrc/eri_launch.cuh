@@ -24,6 +24,7 @@ struct LaunchArgs {
   const double* rootbuf = nullptr;     // precomputed roots [record's base + (b*npij + a)*2*NR]
   const long long* rootbase = nullptr;  // per record of this launch: its base in rootbuf
   int nsplit = 1;       // groups sharing one quartet's primitive quartets (power of two; prim_split)
+  int chain = 0;        // kChainPrev, kChainNext (chain.cuh)
 };
 
 // Device scratch for classes whose transform buffers live in global memory: returns a buffer
@@ -76,10 +77,8 @@ cudaError_t launch_eri(const LaunchArgs& a) {
     scratch = class_scratch(sizeof(double) * (size_t)SH::GBUF_PER_BLOCK * (size_t)blocks);
     if (!scratch) return cudaErrorMemoryAllocation;
   }
-  kern<<<(unsigned)blocks, SH::BLOCK, SH::SMEM_BYTES, a.stream>>>(a.recs, a.nrec, a.pairs, a.prims, a.out,
-                                                                   a.st, a.expcutoff, a.rys, scratch, a.prim_eps,
-                                                                   a.rootbuf, a.rootbase, a.nsplit);
-  return cudaGetLastError();
+  return chain_launch(kern, (unsigned)blocks, SH::BLOCK, SH::SMEM_BYTES, a.stream, a.chain, a.recs, a.nrec, a.pairs,
+                      a.prims, a.out, a.st, a.expcutoff, a.rys, scratch, a.prim_eps, a.rootbuf, a.rootbase, a.nsplit);
 }
 
 template <int N, class F>

@@ -139,7 +139,8 @@ __global__ void __launch_bounds__(splitcoop_dims(LI, LJ, LK, LL, ACC).BLOCK, spl
     eri_splitcoop_kernel(const QuartetRec* __restrict__ recs, int nrec, const ShellPair* __restrict__ pairs,
                          const PrimPair* __restrict__ prims, double* __restrict__ out,
                          const __grid_constant__ StrideSet sts, double expcutoff, const __grid_constant__ RysTable rys, double prim_eps,
-                         const double* __restrict__ rootbuf, const long long* __restrict__ rootbase) {
+                         const double* __restrict__ rootbuf, const long long* __restrict__ rootbase, int chain, int nblocks) {
+  if (chain_begin(chain, nblocks)) return;
   using SH = EriShape<LI, LJ, LK, LL, true, double, ACC, kSplitCoopRegs>;
   constexpr SplitCoopDims D = splitcoop_dims(LI, LJ, LK, LL, ACC);
   static_assert(D.ok && splitcoop_violation<LI, LJ, LK, LL, ACC>() == 0,
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(splitcoop_dims(LI, LJ, LK, LL, ACC).BLOCK, spl
   LaneTuples<SH> lt;
   decode_tuples<SH, LJ, LK, LL>(lt, lane);
 
-  for (int q = (int)blockIdx.x * SH::Q + group; q < nrec; q += (int)gridDim.x * SH::Q) {
+  for (int q = (int)blockIdx.x * SH::Q + group; q < nrec; q += nblocks * SH::Q) {
     const QuartetRec rec = recs[q];
     const double* rb = rootbuf ? rootbuf + rootbase[q] : nullptr;
     const ShellPair pij = pairs[rec.pij];
@@ -332,10 +333,8 @@ cudaError_t launch_splitcoop(const LaunchArgs& a) {
   long long blocks = ((long long)a.nrec + SH::Q - 1) / SH::Q;
   const long long cap = a.max_blocks > 0 ? a.max_blocks : (long long)device_sm_count() * 32;
   if (blocks > cap) blocks = cap;
-  kern<<<(unsigned)blocks, SH::BLOCK, D.SMEM_BYTES, a.stream>>>(a.recs, a.nrec, a.pairs, a.prims, a.out, a.st,
-                                                                a.expcutoff, a.rys, a.prim_eps, a.rootbuf,
-                                                                a.rootbase);
-  return cudaGetLastError();
+  return chain_launch(kern, (unsigned)blocks, SH::BLOCK, D.SMEM_BYTES, a.stream, a.chain, a.recs, a.nrec, a.pairs,
+                      a.prims, a.out, a.st, a.expcutoff, a.rys, a.prim_eps, a.rootbuf, a.rootbase);
 }
 
 }  // namespace cintx

@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "chain.cuh"
 #include "common.h"
 
 struct CINTOpt;  // the library's optimizer handle (defined below as cintx::Opt)
@@ -166,7 +167,7 @@ cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const Quartet
                          const ShellPair* pairs, const PrimPair* prims, double* out, const StrideSet& st,
                          double expcutoff, const RysTable& rys, cudaStream_t stream, bool fp32 = false,
                          double prim_eps = 0.0, int variant = 0, const double* rootbuf = nullptr,
-                         const long long* rootbase = nullptr, int nsplit = 1);
+                         const long long* rootbase = nullptr, int nsplit = 1, int chain = 0);
 // Which quartets of one launch share their primitive quartets over several lane groups.  A group's
 // lanes walk a quartet's primitive quartets one after another, so a launch lasts at least as long as
 // its largest quartet (4096 primitive quartets of two contracted s pairs: 1.2 ms on one lane).  `work`
@@ -187,58 +188,6 @@ PrimSplit prim_split(int li, int lj, int lk, int ll, double work, long long nrec
 // share a quartet.
 PrimSplit prim_split(int lanes, int most, double resident, double work, long long nrec, double pmax);
 
-// Side streams and events of one forked list of independent launches (host_plan.cpp).  Sets are kept
-// per device in a free list: a call takes one while it queues its launches and gives it back, so there
-// are as many as threads ever queued at once, and no call records an event that another one is still
-// to wait for.
-constexpr int kSideStreams = 7;
-struct SideStreams {
-  cudaStream_t s[kSideStreams];
-  cudaEvent_t fork, join[kSideStreams];
-};
-SideStreams* take_side_streams(int dev);  // nullptr: none could be made
-void give_side_streams(int dev, SideStreams* r);
-
-// Spreads independent launches over a stream and side streams: launches go where the least work has
-// gone so far; the side streams start after the stream's earlier work, and join() makes it wait for them.
-// Without side streams everything runs on the stream, in order.
-class Fork {
- public:
-  Fork(cudaStream_t stream, SideStreams* side, int nside) : stream_(stream), side_(side), n_(side ? nside : 0) {
-    if (n_ > kSideStreams) n_ = kSideStreams;
-    if (n_ > 0) err_ = cudaEventRecord(side_->fork, stream_);
-  }
-  // the stream for a launch of `load` work; keep: the stream itself
-  cudaStream_t next(double load, bool keep = false) {
-    int b = 0;
-    for (int i = 1; i <= n_ && !keep; ++i)
-      if (load_[i] < load_[b]) b = i;
-    load_[b] += load;
-    if (b == 0) return stream_;
-    if (!used_[b] && err_ == cudaSuccess) err_ = cudaStreamWaitEvent(side_->s[b - 1], side_->fork, 0);
-    used_[b] = true;
-    return side_->s[b - 1];
-  }
-  cudaError_t error() const { return err_; }
-  cudaError_t join() {
-    for (int b = 1; b <= n_; ++b)
-      if (used_[b]) {
-        const cudaError_t r1 = cudaEventRecord(side_->join[b - 1], side_->s[b - 1]);
-        const cudaError_t r2 = cudaStreamWaitEvent(stream_, side_->join[b - 1], 0);
-        if (err_ == cudaSuccess) err_ = r1 != cudaSuccess ? r1 : r2;
-      }
-    n_ = 0;
-    return err_;
-  }
-
- private:
-  cudaStream_t stream_;
-  SideStreams* side_;
-  int n_;
-  double load_[kSideStreams + 1] = {0};
-  bool used_[kSideStreams + 1] = {false};
-  cudaError_t err_ = cudaSuccess;
-};
 // Learned Rys roots (rysnet.cu) of order n at count device points: out[p*2n + f], status[p]
 // (0 refined, 1 table fallback, 2 closed form), asynchronous on stream.
 cudaError_t rys_learned_eval(const float* d_params, const RysTable& rys, int n, const double* d_x, long long count,

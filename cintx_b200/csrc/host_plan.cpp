@@ -40,49 +40,12 @@ cudaError_t launch_block_absmax_sqrt(const QuartetRec* recs, long long nrec, con
                                      double* q, cudaStream_t stream);
 cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
                                const double* dm, int nao, double* A, double* B, cudaStream_t stream,
-                               int ni, int nj, int nk, int nl);
+                               int ni, int nj, int nk, int nl, int chain);
 cudaError_t launch_symmetrize(const double* X, double* M, int n, cudaStream_t stream);
 cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
                               double* eri, int mode, long long nao, int ni, int nj, int nk, int nl,
-                              cudaStream_t stream);
+                              cudaStream_t stream, int chain);
 }
-
-namespace cintx {
-
-static std::mutex g_side_mu;
-static std::map<int, std::vector<SideStreams*>> g_side;
-
-SideStreams* take_side_streams(int dev) {
-  {
-    std::lock_guard<std::mutex> lk(g_side_mu);
-    std::vector<SideStreams*>& v = g_side[dev];
-    if (!v.empty()) {
-      SideStreams* r = v.back();
-      v.pop_back();
-      return r;
-    }
-  }
-  SideStreams* r = new SideStreams();
-  bool ok = cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming) == cudaSuccess;
-  for (int i = 0; i < kSideStreams && ok; ++i)
-    ok = cudaStreamCreateWithFlags(&r->s[i], cudaStreamNonBlocking) == cudaSuccess &&
-         cudaEventCreateWithFlags(&r->join[i], cudaEventDisableTiming) == cudaSuccess;
-  if (ok) return r;
-  if (r->fork) cudaEventDestroy(r->fork);
-  for (int i = 0; i < kSideStreams; ++i) {
-    if (r->s[i]) cudaStreamDestroy(r->s[i]);
-    if (r->join[i]) cudaEventDestroy(r->join[i]);
-  }
-  delete r;
-  cudaGetLastError();  // the caller runs on one stream instead
-  return nullptr;
-}
-void give_side_streams(int dev, SideStreams* r) {
-  std::lock_guard<std::mutex> lk(g_side_mu);
-  g_side[dev].push_back(r);
-}
-
-}  // namespace cintx
 
 using namespace cintx;
 
@@ -633,9 +596,10 @@ static bool segment_scratch(const CintxPlan* p, const Segment& sg) {
   return sg.groups() == 1 && class_needs_scratch(sg.li, sg.lj, sg.lk, sg.ll, p->sph, sg.variant);
 }
 
-// Runs one segment's class kernel; gen: its records are written first (else they are there already).
+// Runs one segment's class kernel; gen: its records are written first (else they are there already);
+// chain: its place in a chain of launches (chain.cuh).
 static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStream_t stream, DeviceState* ds,
-                       ThreadScratch* ts, bool gen) {
+                       ThreadScratch* ts, bool gen, int chain = 0) {
   const Opt* o = p->opt;
   const QuartetRec* recs;
   long long nrec;
@@ -669,7 +633,7 @@ static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStr
     cudaError_t e = launch_class(sg.li, sg.lj, sg.lk, sg.ll, p->sph, recs + r0, nr, o->d_pairs, o->d_prims,
                                  out_dev + sg.out_off, sg.strides >= 0 ? p->stride_sets[sg.strides] : one_stride(sg.st), sg.expcutoff, ds->rys, stream, sg.fp32, sg.prim_eps,
                                  sg.variant, rb ? p->d_rootbuf : nullptr, rb ? p->d_rootbase + sg.rec0 + r0 : nullptr,
-                                 sg.groups());
+                                 sg.groups(), chain);
     if (e != cudaSuccess) {
       set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("kernel launch failed: ") + cudaGetErrorString(e));
       return CINTX_STATUS_EXECUTION_FAILED;
@@ -679,55 +643,64 @@ static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStr
   return CINTX_STATUS_SUCCESS;
 }
 
-// Runs one chunk's segments on `stream`, each followed by after(segment, its stream) where given.
+// Runs one chunk's segments on `stream`, and after(segment, its place in a chain) for each where given.
 // Segments are independent (disjoint records and output blocks), and most launches of a molecule of
-// some ten atoms fill a fraction of the chip for some ten microseconds, so they are spread over the
-// caller's stream and side streams that start after its earlier work and that it waits for, largest
-// segments first.  Classes that keep their transform buffers in the thread's one device scratch stay
-// on the caller's stream, in order.  A stream under capture is used alone, and so is the caller's
-// stream for chunks whose segments average over kForkFlops: those launches fill the chip by
-// themselves, and a segment's J/K contraction finds less of its blocks in L2 when others run beside it
-// (J/K of 120 s/p/d/f atoms, 2e10 flops a segment: 309 ms in order, 315 forked; all quartets of 3 atoms
-// 1.37 ms in order, 0.29 forked; 24-atom s/p/d/f sweep, 3e8 a segment, 13.0 and 6.9 ms).
-constexpr double kForkFlops = 4e9;
+// some ten atoms fill a fraction of the chip for some ten microseconds, so they are one chain of launches
+// that overlap (chain.cuh), and the launches of after() are a second one behind it.  Classes that keep
+// their transform buffers in the thread's one device scratch start only when all ahead of them is done.
+// A stream under capture gets plain launches in order.  Every Schwarz-surviving quartet, and J and K, in plain
+// launches and so: 3 atoms s/p/d 0.39 -> 0.10 and 0.54 -> 0.14 ms, 24 s/p/d/f 8.9 -> 4.9 and 10.7 -> 6.1,
+// 120 s/p/d/f 228.9 -> 222.4 and 277.6 -> 269.2.
 static int run_chunk(CintxPlan* p, const Chunk& ch, double* out_dev, cudaStream_t stream, DeviceState* ds,
-                     ThreadScratch* ts, const std::function<int(const Segment&, cudaStream_t)>& after) {
+                     ThreadScratch* ts, const std::function<int(const Segment&, int)>& after) {
   const int n = (int)ch.segs.size();
-  // one launch writes the whole chunk's records, ahead of the fork
+  // one launch writes the whole chunk's records, ahead of the chain
   int rc = gen_records(p, ch.segs.data(), ch.segs.data() + n, stream, ts);
   if (rc) return rc;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  SideStreams* side = nullptr;
-  double total = 0;
-  for (const Segment& sg : ch.segs) total += sg.flops;
-  if (n > 1 && total < kForkFlops * n) {
-    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) cudaGetLastError();  // used alone, as it is
-    else if (cap == cudaStreamCaptureStatusNone) side = take_side_streams(ds->dev);
+  bool chained = n > 1;
+  if (chained) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) cudaGetLastError();  // plain launches, as it is
+    chained = cap == cudaStreamCaptureStatusNone;
   }
-  if (!side) {
+  if (!chained) {
     for (const Segment& sg : ch.segs) {
       if ((rc = run_segment(p, sg, out_dev, stream, ds, ts, false))) return rc;
-      if (after && (rc = after(sg, stream))) return rc;
+      if (after && (rc = after(sg, 0))) return rc;
     }
     return CINTX_STATUS_SUCCESS;
   }
-  std::vector<int> idx(n);
-  std::iota(idx.begin(), idx.end(), 0);
-  std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return ch.segs[a].cost() > ch.segs[b].cost(); });
-  Fork fork(stream, side, n - 1);
-  for (int i : idx) {
-    const Segment& sg = ch.segs[i];
-    cudaStream_t st = fork.next(sg.cost(), segment_scratch(p, sg));
-    if (fork.error() != cudaSuccess) break;
-    if ((rc = run_segment(p, sg, out_dev, st, ds, ts, false)) || (after && (rc = after(sg, st)))) break;
+  // largest first; where there are classes with device scratch, each of them at the head of a link that
+  // waits for all ahead of it, and the others dealt out over these links by the time that they take
+  std::vector<int> by_cost(n);
+  std::iota(by_cost.begin(), by_cost.end(), 0);
+  std::stable_sort(by_cost.begin(), by_cost.end(), [&](int a, int b) { return ch.segs[a].cost() > ch.segs[b].cost(); });
+  std::vector<std::vector<int>> links;
+  for (int i : by_cost)
+    if (segment_scratch(p, ch.segs[i])) links.push_back({i});
+  if (links.empty()) links.emplace_back();
+  std::vector<double> load(links.size(), 0.0);
+  for (int i : by_cost) {
+    if (segment_scratch(p, ch.segs[i])) continue;
+    auto share = [&](size_t k) { return links[k].empty() ? 0.0 : load[k] / ch.segs[links[k][0]].cost(); };
+    size_t best = 0;
+    for (size_t k = 1; k < links.size(); ++k)
+      if (share(k) < share(best)) best = k;
+    load[best] += ch.segs[i].cost();
+    links[best].push_back(i);
   }
-  const cudaError_t e = fork.join();
-  give_side_streams(ds->dev, side);
-  if (!rc && e != cudaSuccess) {
-    set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("side streams failed: ") + cudaGetErrorString(e));
-    rc = CINTX_STATUS_EXECUTION_FAILED;
+  int k = 0;
+  for (const auto& link : links)
+    for (size_t j = 0; j < link.size(); ++j) {
+      const int chain = (j > 0 ? kChainPrev : 0) | (j + 1 < link.size() ? kChainNext : 0);
+      if ((rc = run_segment(p, ch.segs[link[j]], out_dev, stream, ds, ts, false, chain))) return rc;
+    }
+  for (int i : by_cost) {
+    if (!after) break;
+    if ((rc = after(ch.segs[i], (k > 0 ? kChainPrev : 0) | (k + 1 < n ? kChainNext : 0)))) return rc;
+    ++k;
   }
-  return rc;
+  return CINTX_STATUS_SUCCESS;
 }
 
 static int exec_prepare(CintxPlan* p, double* out_dev, void* stream_, cudaStream_t* stream, DeviceState** ds,
@@ -1084,11 +1057,11 @@ int cintx_plan_execute_ao(CintxPlan* p, int aosym, double* eri, int64_t len, voi
   ThreadScratch* ts;
   int rc;
   if ((rc = device_state(&ds)) || (rc = thread_scratch(&ts, 0, 0))) return rc;
-  auto scatter = [&](const Segment& sg, cudaStream_t st) -> int {
+  auto scatter = [&](const Segment& sg, int chain) -> int {
     const QuartetRec* recs = p->d_recs + sg.rec0;
     if (launch_scatter_ao(recs, sg.nrec, p->d_pao, p->d_stage, eri, aosym, nao, nsph_or_cart(sg.li, p->sph),
                           nsph_or_cart(sg.lj, p->sph), nsph_or_cart(sg.lk, p->sph), nsph_or_cart(sg.ll, p->sph),
-                          st) == cudaSuccess)
+                          stream, chain) == cudaSuccess)
       return CINTX_STATUS_SUCCESS;
     set_error(CINTX_STATUS_EXECUTION_FAILED, "scatter launch failed");
     return CINTX_STATUS_EXECUTION_FAILED;
@@ -1147,10 +1120,10 @@ int cintx_plan_jk(CintxPlan* p, const double* dm, int nao, double* vj, double* v
   ThreadScratch* ts;
   int rc;
   if ((rc = device_state(&ds)) || (rc = thread_scratch(&ts, 0, 0))) return rc;
-  auto contract = [&](const Segment& sg, cudaStream_t st) -> int {
-    if (launch_jk_contract(p->d_recs + sg.rec0, sg.nrec, p->d_pao, p->d_stage, dm, nao, A, Bk, st,
+  auto contract = [&](const Segment& sg, int chain) -> int {
+    if (launch_jk_contract(p->d_recs + sg.rec0, sg.nrec, p->d_pao, p->d_stage, dm, nao, A, Bk, stream,
                            nsph_or_cart(sg.li, p->sph), nsph_or_cart(sg.lj, p->sph), nsph_or_cart(sg.lk, p->sph),
-                           nsph_or_cart(sg.ll, p->sph)) == cudaSuccess)
+                           nsph_or_cart(sg.ll, p->sph), chain) == cudaSuccess)
       return CINTX_STATUS_SUCCESS;
     set_error(CINTX_STATUS_EXECUTION_FAILED, "J/K contraction launch failed");
     return CINTX_STATUS_EXECUTION_FAILED;

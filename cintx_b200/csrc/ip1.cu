@@ -209,7 +209,7 @@ size_t ip1_image_bytes(const Ip1Work& W, size_t* o_prims, size_t* o_recs) {
 // `host` (kept by the caller until the stream has consumed it) and launches every class group on
 // `stream`, writing into out_dev.
 int ip1_launch(const Ip1Work& W, bool sph, int nsh, const Basis& B, char* dev, char* host, double* out_dev,
-               cudaStream_t stream, const RysTable& rys, int devid, int64_t* nlaunch) {
+               cudaStream_t stream, const RysTable& rys, int64_t* nlaunch) {
   size_t o_prims, o_recs;
   const size_t total = ip1_image_bytes(W, &o_prims, &o_recs);
   memcpy(host, W.pairs.data(), sizeof(ShellPair) * W.pairs.size());
@@ -264,36 +264,29 @@ int ip1_launch(const Ip1Work& W, bool sph, int nsh, const Basis& B, char* dev, c
     return CINTX_STATUS_EXECUTION_FAILED;
   }
   const double cutoff = nsh == 4 ? expcutoff_2e(B.env.data()) : expcutoff_3c(B.env.data());
-  // the launches are independent: largest first over the stream and side streams (as plan chunks)
-  SideStreams* side = launches.size() > 1 ? take_side_streams(devid) : nullptr;
+  // the launches are independent: one chain (chain.cuh)
   int rc = CINTX_STATUS_SUCCESS;
-  {
-    Fork fork(stream, side, (int)launches.size() - 1);
-    for (const Launch& L : launches) {
-      const Ip1Work::Key& k = *L.key;
-      Ip1Args a{};
-      a.pairs = (const ShellPair*)dev;
-      a.prims = (const PrimPair*)(dev + o_prims);
-      a.out = out_dev;
-      a.st = order_strides(k.e);
-      a.scomp = k.e[0] * k.e[1] * k.e[2] * k.e[3];
-      a.expcutoff = cutoff;
-      a.rys = rys;
-      a.nsplit = L.nsplit;
-      a.stream = fork.next(L.work + 3e7);
-      e = fork.error();
-      for (size_t s0 = 0; s0 < L.nrec && e == cudaSuccess; s0 += (size_t)1 << 30) {
-        a.recs = (const QuartetRec*)(dev + o_recs) + L.rec0 + s0;
-        a.nrec = (int)std::min<size_t>(L.nrec - s0, (size_t)1 << 30);
-        e = dispatch_ip1(k.li, k.lj, k.lk, k.ll, sph, a);
-      }
-      if (e != cudaSuccess) break;
-      ++*nlaunch;
+  for (size_t k = 0; k < launches.size() && e == cudaSuccess; ++k) {
+    const Launch& L = launches[k];
+    const Ip1Work::Key& key = *L.key;
+    Ip1Args a{};
+    a.pairs = (const ShellPair*)dev;
+    a.prims = (const PrimPair*)(dev + o_prims);
+    a.out = out_dev;
+    a.st = order_strides(key.e);
+    a.scomp = key.e[0] * key.e[1] * key.e[2] * key.e[3];
+    a.expcutoff = cutoff;
+    a.rys = rys;
+    a.nsplit = L.nsplit;
+    a.stream = stream;
+    a.chain = (k ? kChainPrev : 0) | (k + 1 < launches.size() ? kChainNext : 0);
+    for (size_t s0 = 0; s0 < L.nrec && e == cudaSuccess; s0 += (size_t)1 << 30) {
+      a.recs = (const QuartetRec*)(dev + o_recs) + L.rec0 + s0;
+      a.nrec = (int)std::min<size_t>(L.nrec - s0, (size_t)1 << 30);
+      e = dispatch_ip1(key.li, key.lj, key.lk, key.ll, sph, a);
     }
-    const cudaError_t ej = fork.join();
-    if (e == cudaSuccess) e = ej;
+    ++*nlaunch;
   }
-  if (side) give_side_streams(devid, side);
   if (e != cudaSuccess) {
     set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("derivative kernel launch failed: ") + cudaGetErrorString(e));
     rc = CINTX_STATUS_EXECUTION_FAILED;
@@ -333,7 +326,7 @@ int ip1_eval(int nsh, double* out, bool to_host, const int* shls, int64_t n, boo
   double* dout = to_host ? (double*)(dev + image) : out;
   if (to_host) cudaMemsetAsync(dout, 0, outb, ts->stream);
   int64_t nlaunch = 0;
-  if ((rc = ip1_launch(W, sph, nsh, B, dev, host, dout, ts->stream, ds->rys, ds->dev, &nlaunch))) return rc;
+  if ((rc = ip1_launch(W, sph, nsh, B, dev, host, dout, ts->stream, ds->rys, &nlaunch))) return rc;
   if (to_host) cudaMemcpyAsync(out, dout, outb, cudaMemcpyDeviceToHost, ts->stream);
   ts->launches += nlaunch;
   const cudaError_t e = cudaStreamSynchronize(ts->stream);

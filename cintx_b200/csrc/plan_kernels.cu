@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "chain.cuh"
 #include "common.h"
 
 __global__ void gen_tile_quartets(const int* __restrict__ rows, const int* __restrict__ cols,
@@ -180,10 +181,12 @@ __device__ __forceinline__ double pair_weight(const int2& p) { return p.y < 0 ? 
 // Each (row, column) pair of a block reduces its sum first and adds it with one atomic.
 __global__ void jk_contract_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
                                    const double* __restrict__ out, const double* __restrict__ dm, int nao,
-                                   double* __restrict__ A, double* __restrict__ B, int ni, int nj, int nk, int nl) {
+                                   double* __restrict__ A, double* __restrict__ B, int ni, int nj, int nk, int nl,
+                                   int chain, int nblocks) {
+  if (chain_begin(chain, nblocks)) return;
   const int lane = threadIdx.x & 31;
   for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < nrec;
-       r += ((long long)gridDim.x * blockDim.x) >> 5) {
+       r += ((long long)nblocks * blockDim.x) >> 5) {
     const QuartetRec rec = recs[r];
     const int2 ab = pao[rec.pij], cd = pao[rec.pkl];
     const int i0 = ab.x, j0 = pair_ao(ab), k0 = cd.x, l0 = pair_ao(cd);
@@ -254,12 +257,13 @@ __global__ void jk_contract_kernel(const QuartetRec* __restrict__ recs, long lon
 template <int MODE>
 __global__ void scatter_ao_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
                                   const double* __restrict__ out, double* __restrict__ eri, long long nao, SmallDiv ni, SmallDiv nj, SmallDiv nk,
-                                  SmallDiv nl, int G) {
+                                  SmallDiv nl, int G, int chain, int nblocks) {
+  if (chain_begin(chain, nblocks)) return;
   const int g = threadIdx.x & (G - 1);
   const long long npair = nao * (nao + 1) / 2, n2 = nao * nao;
   const unsigned n = ni.d * nj.d * nk.d * nl.d;
   const unsigned sj = ni.d, sk = ni.d * nj.d, sl = ni.d * nj.d * nk.d;
-  const long long ngroups = (long long)gridDim.x * blockDim.x / G;
+  const long long ngroups = (long long)nblocks * blockDim.x / G;
   for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G; r < nrec; r += ngroups) {
     const QuartetRec rec = recs[r];
     const int2 ab = pao[rec.pij], cd = pao[rec.pkl];
@@ -384,7 +388,8 @@ __global__ void __launch_bounds__(32 * kJkWarps)
     jk_contract_group_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
                              const double* __restrict__ out,
                              const double* __restrict__ dm, int nao, double* __restrict__ A, double* __restrict__ B,
-                             SmallDiv di_, SmallDiv dj_, int G, int run) {
+                             SmallDiv di_, SmallDiv dj_, int G, int run, int chain, int nblocks) {
+  if (chain_begin(chain, nblocks)) return;
   constexpr int NP = NK <= 1 ? 1 : NK <= 2 ? 2 : NK <= 4 ? 4 : NK <= 8 ? 8 : 16;
   constexpr int NKL = NK + NL;
   extern __shared__ double sm[];
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(32 * kJkWarps)
   double* s_aij = s_akl + NK * NL;
   double* s_t = s_aij + nij;  // [2 * NKL][nij]: sums over l with D[j,l], over k with D[j,k]; with D[i,l], D[i,k]
   const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
-  const long long ngroups = (long long)gridDim.x * blockDim.x / G;
+  const long long ngroups = (long long)nblocks * blockDim.x / G;
   for (long long base = gid * run; base < nrec; base += ngroups * run) {
     const long long rend = base + run < nrec ? base + run : nrec;
     int cur = -1;  // the (ij) pair whose A[i,j] sums s_aij holds
@@ -530,10 +535,11 @@ template <int NI, int NK>
 __global__ void __launch_bounds__(128)
     jk_contract_thread_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
                               const double* __restrict__ out, const double* __restrict__ dm, int nao,
-                              double* __restrict__ A, double* __restrict__ B, int nj) {
+                              double* __restrict__ A, double* __restrict__ B, int nj, int chain, int nblocks) {
+  if (chain_begin(chain, nblocks)) return;
   constexpr int NP = NI <= 1 ? 1 : NI <= 4 ? 4 : NI <= 8 ? 8 : 16;
   const int lane = threadIdx.x & 31;
-  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long stride = (long long)nblocks * blockDim.x;
   // whole warps run (lanes past the end repeat the last record with weight 0 and store nothing)
   for (long long r0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) - lane; r0 < nrec; r0 += stride) {
     const bool on = r0 + lane < nrec;
@@ -664,7 +670,7 @@ static size_t jk_group_smem(int nij, int nk, int nl) {
 template <int NK, int NL>
 static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
                                    const double* dm, int nao, double* A, double* B,
-                                   cudaStream_t stream, int ni, int nj) {
+                                   cudaStream_t stream, int ni, int nj, int chain) {
   const int G = jk_group_lanes(ni * nj);
   const size_t smem = jk_group_smem(ni * nj, NK, NL);
   auto kern = jk_contract_group_kernel<NK, NL>;
@@ -683,17 +689,17 @@ static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const
   const long long per_block = 32LL * kJkWarps / G * run;
   long long blocks = (nrec + per_block - 1) / per_block;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
-  kern<<<(unsigned)blocks, 32 * kJkWarps, smem, stream>>>(recs, nrec, pao, out, dm, nao, A, B, small_divisor(ni),
-                                                          small_divisor(nj), G, run);
-  return cudaGetLastError();
+  return chain_launch(kern, (unsigned)blocks, 32 * kJkWarps, smem, stream, chain, recs, nrec, pao, out, dm, nao, A, B,
+                      small_divisor(ni), small_divisor(nj), G, run);
 }
 
 template <int NI, int NK>
 static cudaError_t launch_jk_thread(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
-                                    const double* dm, int nao, double* A, double* B, cudaStream_t stream, int nj) {
+                                    const double* dm, int nao, double* A, double* B, cudaStream_t stream, int nj,
+                                    int chain) {
   const long long blocks = std::min((nrec + 127) / 128, 148LL * 64);
-  jk_contract_thread_kernel<NI, NK><<<(unsigned)blocks, 128, 0, stream>>>(recs, nrec, pao, out, dm, nao, A, B, nj);
-  return cudaGetLastError();
+  return chain_launch(jk_contract_thread_kernel<NI, NK>, (unsigned)blocks, 128, 0, stream, chain, recs, nrec, pao, out,
+                      dm, nao, A, B, nj);
 }
 
 // One class segment, blocks ni x nj x nk x nl.  Small kets (nl = 1, nk <= 3) take a thread per quartet
@@ -702,15 +708,15 @@ static cudaError_t launch_jk_thread(const QuartetRec* recs, long long nrec, cons
 // functions: the sums of one lane no longer fit registers) keep the general kernel.
 cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
                                const double* dm, int nao, double* A, double* B, cudaStream_t stream,
-                               int ni, int nj, int nk, int nl) {
+                               int ni, int nj, int nk, int nl, int chain) {
   if (nrec <= 0) return cudaSuccess;
 #define CINTX_JK_THREAD(I, K) \
-  if (ni == I && nk == K && nl == 1) return launch_jk_thread<I, K>(recs, nrec, pao, out, dm, nao, A, B, stream, nj);
+  if (ni == I && nk == K && nl == 1) return launch_jk_thread<I, K>(recs, nrec, pao, out, dm, nao, A, B, stream, nj, chain);
   CINTX_JK_THREAD(1, 1) CINTX_JK_THREAD(3, 1) CINTX_JK_THREAD(5, 1) CINTX_JK_THREAD(6, 1) CINTX_JK_THREAD(7, 1)
   CINTX_JK_THREAD(9, 1) CINTX_JK_THREAD(3, 3) CINTX_JK_THREAD(5, 3) CINTX_JK_THREAD(6, 3) CINTX_JK_THREAD(7, 3)
 #undef CINTX_JK_THREAD
 #define CINTX_JK(K, L) \
-  if (nk == K && nl == L) return launch_jk_group<K, L>(recs, nrec, pao, out, dm, nao, A, B, stream, ni, nj);
+  if (nk == K && nl == L) return launch_jk_group<K, L>(recs, nrec, pao, out, dm, nao, A, B, stream, ni, nj, chain);
   if (jk_group_smem(ni * nj, nk, nl) <= kJkSmem) {
     CINTX_JK(1, 1) CINTX_JK(3, 1) CINTX_JK(3, 3)  // (1, 1) and (3, 1): cartesian g first shells
     CINTX_JK(5, 1) CINTX_JK(5, 3) CINTX_JK(5, 5)
@@ -722,23 +728,21 @@ cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int
 #undef CINTX_JK
   long long blocks = (nrec * 32 + 255) / 256;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
-  jk_contract_kernel<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, pao, out, dm, nao, A, B, ni, nj, nk, nl);
-  return cudaGetLastError();
+  return chain_launch(jk_contract_kernel, (unsigned)blocks, 256, 0, stream, chain, recs, nrec, pao, out, dm, nao, A, B,
+                      ni, nj, nk, nl);
 }
 
 cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
                               double* eri, int mode, long long nao, int ni, int nj, int nk, int nl,
-                              cudaStream_t stream) {
+                              cudaStream_t stream, int chain) {
   if (nrec <= 0) return cudaSuccess;
   int G = 1;
   while (G < 32 && G < ni * nj * nk * nl) G *= 2;
   long long blocks = (nrec * G + 255) / 256;
   if (blocks > 148LL * 64) blocks = 148LL * 64;
   auto kern = mode == 1 ? scatter_ao_kernel<1> : (mode == 4 ? scatter_ao_kernel<4> : scatter_ao_kernel<8>);
-  kern<<<(unsigned)blocks, 256, 0, stream>>>(recs, nrec, pao, out, eri, nao, small_divisor(ni), small_divisor(nj), small_divisor(nk),
-                                             small_divisor(nl),
-                                             G);
-  return cudaGetLastError();
+  return chain_launch(kern, (unsigned)blocks, 256, 0, stream, chain, recs, nrec, pao, out, eri, nao, small_divisor(ni),
+                      small_divisor(nj), small_divisor(nk), small_divisor(nl), G);
 }
 
 cudaError_t launch_symmetrize(const double* X, double* M, int n, cudaStream_t stream) {

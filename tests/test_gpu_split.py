@@ -281,3 +281,40 @@ def test_tuning_a_small_molecule_leaves_larger_ones_their_shapes():
         many.autotune(buf.data_ptr(), chunk=-1, stream=s, reps=1)
         assert many.use_tuned_shapes() == len(lanes) and len(cx.tuned_shapes()) >= 1
         few.close(), many.close()
+
+
+def test_work_behind_a_held_stream_holds_up_no_other():
+    """A list of many classes queued behind a long kernel on one stream, then the same and a plain copy on
+    others: they are done while the first is still held up."""
+    import cintx_b200 as cx
+    import torch
+    mol = contracted([0, 0, 1, 1, 2], [8, 1, 3, 1, 1], 25)
+    i, j = np.tril_indices(mol.nbas)
+    a, b = np.tril_indices(i.size)
+    q = np.stack([i[a], j[a], i[b], j[b]], axis=1).astype(np.int32)
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+        plan = cx.Plan.shells(opt, cx.INT2E, q)
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        outs = [torch.zeros(plan.stats.nintegrals, dtype=torch.float64, device="cuda") for _ in range(2)]
+        torch.cuda.synchronize()
+        for s, o in zip(streams, outs):
+            plan.execute(o.data_ptr(), stream=s.cuda_stream)
+        torch.cuda.synchronize()
+        ref = outs[0].clone()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(1_000_000_000)  # cycles: half a second
+            held = torch.cuda.Event()
+            held.record()
+        for s, o in zip(streams, outs):
+            plan.execute(o.data_ptr(), stream=s.cuda_stream)
+        rest = [torch.cuda.Stream() for _ in range(8)]  # as many as there are hardware queues
+        for s in rest:
+            with torch.cuda.stream(s):
+                ref.clone()
+        for s in streams[1:] + rest:
+            s.synchronize()
+        assert not held.query()
+        torch.cuda.synchronize()
+        assert torch.equal(outs[0], ref) and torch.equal(outs[1], ref)
+        plan.close()
