@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(32 * kJkWarps)
         const double* v = out + rec.out + (on ? ij : 0);
         const double* di = dm + (size_t)(i0 + i) * nao;
         const double* dj = dm + (size_t)(j0 + j) * nao;
-        const double dij = di[j0 + j];
+        const double dij = on ? di[j0 + j] : 0.0;  // not 0 times an infinity in a lane without an element
         double djk[NK], dik[NK], t[NK], u[NK];
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(128)
           sil[i] = fma(x, djk[k], sil[i]);
           wjl = fma(x, dik[i][k], wjl);
         }
-        p[i] = aij;
+        p[i] = on ? aij : 0.0;  // weight 0 times an infinite density is not 0
       }
       if (A) {
         if (one_row) {

@@ -318,3 +318,32 @@ def test_work_behind_a_held_stream_holds_up_no_other():
         torch.cuda.synchronize()
         assert torch.equal(outs[0], ref) and torch.equal(outs[1], ref)
         plan.close()
+
+
+@pytest.mark.parametrize("sph", [True, False])
+def test_j_of_an_infinite_density_element(sph):
+    """An infinite density element makes every element of J infinite that it reaches by a nonzero
+    integral, not NaN: lanes that pad a group or a warp add nothing."""
+    import cintx_b200 as cx
+    import torch
+    mol = contracted([0, 1, 2, 3], [2, 1, 1, 1], 27)
+    l = mol.bas[:, 1].astype(int)
+    nao = int((2 * l + 1 if sph else (l + 1) * (l + 2) // 2).sum())
+    s = torch.cuda.current_stream().cuda_stream
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+        plan = cx.Plan.screened(opt, 0.0, sph=sph)
+        eri = torch.empty(nao ** 4, dtype=torch.float64, device="cuda")
+        plan.execute_ao(eri.data_ptr(), eri.numel(), 1, s)
+        eri = eri.reshape(nao, nao, nao, nao)
+        vj = torch.empty(nao, nao, dtype=torch.float64, device="cuda")
+        n = 0
+        for a in range(nao):
+            b = (7 * a) % nao
+            dm = torch.ones(nao, nao, dtype=torch.float64, device="cuda")
+            dm[a, b] = dm[b, a] = float("inf")
+            plan.jk(dm.data_ptr(), nao, vj.data_ptr(), 0, s)
+            reached = eri[:, :, a, b].abs() > 1e-10  # zeros by symmetry are of either sign, or 0
+            assert vj[reached].isinf().all(), (a, b)
+            n += int(reached.sum())
+        assert n > nao
+        plan.close()
