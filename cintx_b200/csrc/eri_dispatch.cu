@@ -96,18 +96,19 @@ int variant_shape(int li, int lj, int lk, int ll, bool sph, bool fp32, int varia
          variant_regs(variant);
 }
 
-int default_variant(int li, int lj, int lk, int ll) {
+int default_variant(int li, int lj, int lk, int ll, double np) {
   if (li > CINTX_LMAX || !class_valid(li, lj, lk, ll) || default_threads(li, lj, lk, ll) == 1) return 0;
   auto lanes = [&](int v) { return sliced_ok(li, lj, lk, ll, v) ? pick_threads(li, lj, lk, ll, variant_acc(v)) : 0; };
   if (lanes(4) == 2) return 4;
   if (lanes(5) == 2) return 5;
   if (lanes(7) > 0) return 7;
-  for (int v : {11, 10})
-    if (splitcoop_applies(li, lj, lk, ll, v)) return v;
+  if (li >= 3)
+    for (int v : {11, 10})
+      if (splitcoop_applies(li, lj, lk, ll, v)) return v;
   // 256 lanes with more accumulators than 128 registers hold: 255 registers
   const int s = default_threads(li, lj, lk, ll), ntup = ncart(lj) * ncart(lk) * ncart(ll);
-  if ((ntup + s - 1) / s * ncart(li) > 40) return 1;
-  return 0;
+  const int acc = (ntup + s - 1) / s * ncart(li);
+  return acc > 45 || (acc > 40 && np >= 2) ? 1 : 0;
 }
 
 bool class_needs_scratch(int li, int lj, int lk, int ll, bool sph, int variant) {

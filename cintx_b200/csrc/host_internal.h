@@ -198,17 +198,22 @@ int variant_lanes(int li, int lj, int lk, int ll, bool sph, bool fp32, int varia
 // Distinct launch shape of a variant (lanes and register cap), for telling variants apart.
 int variant_shape(int li, int lj, int lk, int ll, bool sph, bool fp32, int variant);
 constexpr int kLaunchVariants = 12;
-// The variant a spherical FP64 launch starts with when nothing was tuned, by the class's size alone:
+// The variant a spherical FP64 launch of quartets of np primitive quartets (their mean) starts with when
+// nothing was tuned, by the class's size and np alone:
 //   at most 48 functions         the default shape, one lane (default_acc);
 //   2 lanes of 32, or else of 48 the sliced shapes with their roots unrolled (4, 5): every lane its own
 //                                recurrences in registers, no barrier per primitive quartet;
 //   up to 4 lanes of 48          the same with the roots rolled (7), tables of at most 72 doubles;
-//   64 lanes or more             split horizontal transfers (11: 24 accumulators per lane, else 10: 12);
-//   over 40 accumulators a lane  (256 lanes, several g shells) the default shape with 255 registers (1);
+//   64 lanes or more, an f shell split horizontal transfers (11: 24 accumulators per lane, else 10: 12).
+//                                Of (22|22), the one class without, they take 1.03 to 1.17 times the default
+//                                shape's time (3000 quartets of 1, 16 and 81 primitive quartets);
+//   over 40 accumulators a lane  (256 lanes, several g shells) the default shape with 255 registers (1).  With
+//                                45 it pays for the primitive loop only: (42|42) and (44|22) of 1 primitive
+//                                quartet 1.24 and 1.11 times the default shape's time, of 16 0.84 and 0.60;
 //   the rest                     the default shape.
 // All classes of a 120-atom s/p/d/f molecule, one after another: default shapes 274.7 ms, this rule
 // 202.6, the fastest shape of each class as timed by the autotuner 202.1; 3-centre sweep of 40 atoms 3.84,
 // 2.81 and 2.72 ms.
-int default_variant(int li, int lj, int lk, int ll);
+int default_variant(int li, int lj, int lk, int ll, double np);
 
 }  // namespace cintx

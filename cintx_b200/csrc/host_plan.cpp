@@ -491,7 +491,6 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
       p->stride_sets.push_back(order_strides({extent[0], extent[1], extent[2], extent[3]}));
       sg.expcutoff = cutoff;
       sg.rec0 = rec0;
-      if (p->sph) sg.variant = default_variant(k.li, k.lj, k.lk, k.ll);
       ch.segs.push_back(sg);
       seg_work.emplace_back(0.0, 0.0);
       seg_extent = extent;
@@ -511,6 +510,7 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
     const PrimSplit ps = prim_split(sg.li, sg.lj, sg.lk, sg.ll, seg_work[i].first, sg.nrec, seg_work[i].second);
     sg.nsplit = ps.ns;
     sg.work = seg_work[i].first;
+    if (p->sph) sg.variant = default_variant(sg.li, sg.lj, sg.lk, sg.ll, sg.work / (double)sg.nrec);
     if (ps.ns > 1 && ps.pmin > 0) heavy.emplace_back(i, ps.pmin);
   }
   {
@@ -1778,6 +1778,7 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
     if (o->pair_nprim[id] > 0) cls[std::make_pair(o->pair_la[id], o->pair_lb[id])].push_back(id);
   // per class, the pairs whose diagonal quartets share lane groups (prim_split) first
   std::map<std::pair<int, int>, PrimSplit> split;
+  std::map<std::pair<int, int>, double> mean_np;
   auto diag_np = [&](int id) { return (double)o->pair_nprim[id] * (double)o->pair_nprim[id]; };
   for (auto& kv : cls) {
     double work = 0, pmax = 0;
@@ -1790,6 +1791,7 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
     if (ps.ns > 1)
       std::stable_partition(kv.second.begin(), kv.second.end(), [&](int id) { return diag_np(id) >= ps.pmin; });
     split[kv.first] = ps;
+    mean_np[kv.first] = work / (double)kv.second.size();
   }
   const long long cap = 1LL << 25;  // doubles of diagonal blocks per batch
   std::vector<QuartetRec> recs;
@@ -1825,7 +1827,7 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
             const long long q0 = part ? rs : r0, q1 = part ? seg_end[g] : rs;
             if (q1 <= q0) continue;
             ok = launch_class(la, lb, la, lb, true, d_recs + q0, (int)(q1 - q0), o->d_pairs, o->d_prims, d_out, one_stride(st),
-                              ecut, ds->rys, ts->stream, false, 0.0, default_variant(la, lb, la, lb), nullptr, nullptr,
+                              ecut, ds->rys, ts->stream, false, 0.0, default_variant(la, lb, la, lb, mean_np[seg_cls[g]]), nullptr, nullptr,
                               part ? 1 : ps.ns) ==
                  cudaSuccess;
             ts->launches++;
@@ -2125,7 +2127,6 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
       m.prim_eps = p0.prim_eps;
       m.swap = p0.swap;
       m.nsplit = nsplit;
-      if (p->sph && !m.fp32) m.variant = default_variant(m.li, m.lj, m.lk, m.ll);
       m.rec0 = rec;
       m.out_off = 0;
       m.range0 = (int)p->ranges.size();
@@ -2150,6 +2151,7 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
         m.work += (double)(pc.t1 - pc.t0) * piece_np(i);
       }
       m.nranges = (int)p->ranges.size() - m.range0;
+      if (p->sph && !m.fp32) m.variant = default_variant(m.li, m.lj, m.lk, m.ll, m.work / (double)m.nrec);
       rec += m.nrec;
       ch.segs.push_back(m);
     };

@@ -262,7 +262,7 @@ def test_tuning_a_small_molecule_leaves_larger_ones_their_shapes():
     would have run before."""
     import cintx_b200 as cx
     import torch
-    mol = contracted([2, 1, 2, 1], [3, 3, 3, 3], 23)
+    mol = contracted([3, 1, 3, 1], [3, 3, 3, 3], 23)
     q = np.array([[0, 5, 10, 3], [4, 9, 2, 7]], dtype=np.int32)
     s = torch.cuda.current_stream().cuda_stream
     with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
