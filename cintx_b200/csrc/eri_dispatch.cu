@@ -34,11 +34,12 @@ cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const Quartet
 
 constexpr double kSplitLarge = 1024;
 
-PrimSplit prim_split(int lanes, int most, double resident, double work, long long nrec, double pmax) {
+PrimSplit prim_split(int lanes, int most, double resident, double work, long long nrec, double pmax, double least) {
   PrimSplit r;
   if (most <= 1 || nrec <= 0) return r;
   const double share = std::max(work / resident, lanes == 1 ? 16.0 : 4.0);
-  if (pmax < 2 * share) {
+  const double from = std::max(2 * share, least * work / resident);
+  if (pmax < from) {
     if (lanes == 1 && pmax >= kSplitLarge) {
       r.ns = 8;
       r.pmin = kSplitLarge;
@@ -48,15 +49,23 @@ PrimSplit prim_split(int lanes, int most, double resident, double work, long lon
   r.ns = 2;
   while (r.ns < most && r.ns * share < pmax) r.ns *= 2;
   if (lanes == 1 && r.ns == 64) r.ns = 32;  // one-lane teams: at most a warp, or a block
-  r.pmin = (double)nrec * r.ns <= 2 * resident ? 0 : 2 * share;
+  r.pmin = (double)nrec * r.ns <= 2 * resident ? 0 : from;
   if (lanes == 1 && r.pmin > kSplitLarge) r.pmin = kSplitLarge;
   return r;
 }
 
-PrimSplit prim_split(int li, int lj, int lk, int ll, double work, long long nrec, double pmax) {
+PrimSplit prim_split(int li, int lj, int lk, int ll, bool sph, double work, long long nrec, double pmax) {
   const int s = default_threads(li, lj, lk, ll);
-  if (split_max(s) <= 1) return PrimSplit();
-  return prim_split(s, split_max(s), (double)device_sm_count() * 4 * (128 / s), work, nrec, pmax);
+  if (split_max(s) <= 1 || nrec <= 0) return PrimSplit();
+  double least = 2;
+  if (s == 1) {
+    if (ncart(li) * ncart(lj) * ncart(lk) * ncart(ll) > 10) least = 3;
+  } else if (sph) {
+    const int v = default_variant(li, lj, lk, ll, work / (double)nrec);
+    if (variant_sliced(v)) least = 8;
+    else if (variant_splitcoop(v)) least = 3;
+  }
+  return prim_split(s, split_max(s), (double)device_sm_count() * 4 * (128 / s), work, nrec, pmax, least);
 }
 
 static_assert(kNumVariants == kLaunchVariants, "variant count differs between kernel and host headers");

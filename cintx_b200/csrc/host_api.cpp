@@ -745,7 +745,7 @@ static int eval_call(int family, bool sph, double* out, int* dims, int* shls, in
   cudaError_t e = launch_class(ori.li, ori.lj, ori.lk, ori.ll, sph, (const QuartetRec*)(d + off_recs), (int)recs.size(),
                                (const ShellPair*)(d + off_pairs), (const PrimPair*)(d + off_prims),
                                kout, one_stride(st), cutoff, ds->rys, ts->stream, false, 0.0, 0, nullptr, nullptr,
-                               prim_split(ori.li, ori.lj, ori.lk, ori.ll, pwork, (long long)recs.size(), pmax).ns);
+                               prim_split(ori.li, ori.lj, ori.lk, ori.ll, sph, pwork, (long long)recs.size(), pmax).ns);
   if (e != cudaSuccess) {
     set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("kernel launch failed: ") + cudaGetErrorString(e));
     return 0;

@@ -179,14 +179,20 @@ cudaError_t launch_class(int li, int lj, int lk, int ll, bool sph, const Quartet
 // cost as much.  One-lane classes also split quartets of 1024 and more where the launch is even: they
 // are its last to end, and a warp's lanes then run the same quartet (40-atom s/p/d sweep 5.32 -> 5.06 ms
 // with 8 or 32 lanes each; from 256 on 5.23, from 64 on 5.65; J/K of 120 atoms unchanged).
+// Nothing is split under `least` times the even share, which is more where the split form, of the default
+// shape, competes with a faster shape or adds up large blocks.  Lists of equal quartets, split over whole:
+// of sliced classes (default_variant 4, 5, 7) 1.9 times the time at an even share of 1/3 of the quartet (3000
+// quartets of 8 lanes), 1.3 at 1/6, 0.64 at 1/10; of split-transfer classes 1.5 at 0.42, 0.95 at 1/4 and 1/8;
+// of one-lane classes of more than 10 functions 1.2 at 0.4 (30000 quartets of 81), 0.6 at 1/5.
 struct PrimSplit {
   int ns = 1;
   double pmin = 0;
 };
-PrimSplit prim_split(int li, int lj, int lk, int ll, double work, long long nrec, double pmax);
+PrimSplit prim_split(int li, int lj, int lk, int ll, bool sph, double work, long long nrec, double pmax);
 // The rule itself, for groups of `lanes` lanes of which `resident` fit the device and at most `most`
 // share a quartet.
-PrimSplit prim_split(int lanes, int most, double resident, double work, long long nrec, double pmax);
+PrimSplit prim_split(int lanes, int most, double resident, double work, long long nrec, double pmax,
+                     double least = 2);
 
 // Learned Rys roots (rysnet.cu) of order n at count device points: out[p*2n + f], status[p]
 // (0 refined, 1 table fallback, 2 closed form), asynchronous on stream.

@@ -507,7 +507,7 @@ int cintx_plan_shells(CintxPlan** plan, CINTOpt* optp, int family, const int* sh
   }
   for (size_t i = 0; i < ch.segs.size(); ++i) {
     Segment& sg = ch.segs[i];
-    const PrimSplit ps = prim_split(sg.li, sg.lj, sg.lk, sg.ll, seg_work[i].first, sg.nrec, seg_work[i].second);
+    const PrimSplit ps = prim_split(sg.li, sg.lj, sg.lk, sg.ll, p->sph, seg_work[i].first, sg.nrec, seg_work[i].second);
     sg.nsplit = ps.ns;
     sg.work = seg_work[i].first;
     if (p->sph) sg.variant = default_variant(sg.li, sg.lj, sg.lk, sg.ll, sg.work / (double)sg.nrec);
@@ -1787,7 +1787,8 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
       pmax = std::max(pmax, diag_np(id));
     }
     const PrimSplit ps =
-        prim_split(kv.first.first, kv.first.second, kv.first.first, kv.first.second, work, (long long)kv.second.size(), pmax);
+        prim_split(kv.first.first, kv.first.second, kv.first.first, kv.first.second, true, work,
+                   (long long)kv.second.size(), pmax);
     if (ps.ns > 1)
       std::stable_partition(kv.second.begin(), kv.second.end(), [&](int id) { return diag_np(id) >= ps.pmin; });
     split[kv.first] = ps;
@@ -2166,7 +2167,7 @@ static int finish_screened(CintxPlan* p, Opt* o, double ecut, int64_t max_chunk,
         pmax = std::max(pmax, piece_np(i));
       }
       PrimSplit ps;
-      if (!p0.fp32) ps = prim_split(p0.li, p0.lj, p0.lk, p0.ll, work, nq, pmax);
+      if (!p0.fp32) ps = prim_split(p0.li, p0.lj, p0.lk, p0.ll, p->sph, work, nq, pmax);
       if (ps.ns == 1 || ps.pmin <= 0) {
         add_segment(mem, ps.ns);
         continue;
