@@ -6,6 +6,7 @@
 // where violation is shape_violation<Shape>() for eri4c_kernel's shapes and splitcoop_violation
 // for the split-transfer cooperative shapes (variants 10, 11) (0: every shared-memory, scratch,
 // barrier and per-thread index the kernel forms from the shape stays inside its buffer).
+// Kind "split", variant = groups per quartet: the teams of the default shape that share a quartet.
 // Compiled with nvcc as a host program; it launches nothing.
 #include <cstdio>
 
@@ -19,8 +20,29 @@ void row(int li, int lj, int lk, int ll, const char* kind, int v) {
               SH::Q, SH::B_GROUP, SH::SMEM_BYTES, (int)SH::GLOBAL_BUF, shape_violation<SH>());
 }
 
+// Teams of ns groups of the default shape: a whole number of them in the block's 128 threads; one-lane
+// teams a warp's part, a warp or the block; teams of more than a warp and less than the block at named
+// barriers 1 and 2, which the groups themselves must not use; every group's partial block, and in the first
+// group's region the transform buffers, inside a group's shared memory.
+template <class SH>
+int split_violation(int ns) {
+  const int threads = ns * SH::S;
+  if (SH::BLOCK != 128 || SH::Q * SH::S != 128 || SH::Q % ns != 0 || SH::GLOBAL_BUF || SH::IS_SLICE) return 1;
+  if (SH::S == 1) return ns <= 32 || ns == 128 ? 0 : 2;
+  if (threads > 32 && threads < 128 && (SH::S > 32 || 128 / threads > 2)) return 3;
+  if ((SH::SM_BUFA + SH::SM_BUFB) * 8 > SH::B_GROUP || SH::MI * SH::NTUP * 8 > SH::B_GROUP) return 4;
+  return 0;
+}
+
 template <int LI, int LJ, int LK, int LL>
 void shapes_of_class() {
+  static_for<2>([&](auto C) {
+    using SH = EriShape<LI, LJ, LK, LL, decltype(C)::value == 0>;
+    for (int ns = 2; ns <= split_max(SH::S); ns *= 2)
+      if (SH::S > 1 || ns != 64)  // launch_eri refuses teams of two one-lane warps
+        std::printf("%d %d %d %d split %d %d %d %d %d %d %d %d %d\n", LI, LJ, LK, LL, ns, SH::S, SH::LANES, SH::BLOCK,
+                    SH::Q, SH::B_GROUP, SH::SMEM_BYTES, (int)SH::GLOBAL_BUF, split_violation<SH>(ns));
+  });
   row<EriShape<LI, LJ, LK, LL, true>>(LI, LJ, LK, LL, "sph", 0);
   row<EriShape<LI, LJ, LK, LL, false>>(LI, LJ, LK, LL, "cart", 0);
   row<EriShape<LI, LJ, LK, LL, true, float>>(LI, LJ, LK, LL, "fp32", 0);

@@ -80,24 +80,91 @@ def test_derivatives_of_contracted_shells(nsh, sph):
             assert np.allclose(one, got[off[q]:off[q] + one.size], rtol=1e-9, atol=1e-11)
 
 
-@pytest.mark.parametrize("ls", [(0, 0, 0, 0), (1, 0, 1, 0), (2, 0, 2, 0), (2, 1, 2, 1), (2, 2, 2, 2), (3, 2, 3, 2)])
+XMAX = {1: 40, 2: 52, 3: 60, 4: 64, 5: 72, 6: 76, 7: 84, 8: 92, 9: 100}  # end of each order's table
+
+
+def two_centres(ls, x, shift=0.0):
+    """Shells 0 and 1 on one point, 2 and 3 on another, all of exponent 0.7 (a_ij = a_kl = 1.4, rho = 0.7),
+    so that the quartet's only x is the given one; shell 0's atom moved by `shift` along z."""
+    r = float(np.sqrt(x / 0.7))
+    co = [[0.0, 0.0, shift], [0.0, 0.0, 0.0], [0.6 * r, 0.48 * r, 0.64 * r]]
+    return M.build_molecule("ends", co, [[M.ShellSpec(ls[0], [0.7], [1.0])], [M.ShellSpec(ls[1], [0.7], [1.0])],
+                                         [M.ShellSpec(l, [0.7], [1.0]) for l in ls[2:]]])
+
+
+@pytest.mark.parametrize("ls", [(0, 0, 0, 0), (1, 0, 1, 0), (2, 0, 2, 0), (2, 1, 2, 1), (2, 2, 2, 2), (3, 2, 3, 2),
+                                (3, 3, 3, 3), (4, 3, 4, 3), (4, 4, 4, 4)])
 def test_roots_at_the_end_of_the_table(ls):
-    """Quartets whose x lies on, just below and just above the last table interval of their order and
-    the 2^-20 before it where the large-x form starts (xmax of rys_roots, per order 1..6)."""
+    """Quartets whose x lies on, just below and just above the last table interval of their order (1..9)
+    and the 2^-20 before it where the large-x form starts, in single calls and in each launch shape."""
     import cintx_b200 as cx
+    import torch
     from oracle import Restatement
-    n = sum(ls) // 2 + 1
-    xmax = {1: 40, 2: 52, 3: 60, 4: 64, 5: 72, 6: 76}[n]
+    xmax = XMAX[sum(ls) // 2 + 1]
     orc = Restatement()
+    s = torch.cuda.current_stream().cuda_stream
     for eps in (-1e-3, -2.0 ** -20 / xmax, -1e-9, 0.0, 1e-15, 1e-9, 1e-3):
-        a = 0.7  # four equal exponents: a_ij = a_kl = 2a, rho = a, x = a R^2
-        r = float(np.sqrt(xmax * (1.0 + eps) / a))
-        mol = M.build_molecule("ends", [[0.0, 0.0, 0.0], [0.6 * r, 0.48 * r, 0.64 * r]],
-                               [[M.ShellSpec(l, [a], [1.0]) for l in ls[:2]], [M.ShellSpec(l, [a], [1.0]) for l in ls[2:]]])
+        mol = two_centres(ls, xmax * (1.0 + eps))
         q = np.array([[0, 1, 2, 3]], dtype=np.int32)
         ref, _ = orc.int2e_batch(q, mol, sph=True)
         got, _ = cx.int2e_sph(q[0], mol.atm, mol.bas, mol.env)
         assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max() + 1e-15, (ls, eps)
+        if sum(ls) not in (10, 12):  # (32|32), (33|33): sliced and split-transfer shapes exist
+            continue
+        with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+            plan = cx.Plan.shells(opt, cx.INT2E, q)
+            out = torch.empty(plan.stats.nintegrals, dtype=torch.float64, device="cuda")
+            for v in range(12):
+                plan.set_shape(v)
+                plan.execute(out.data_ptr(), stream=s)
+                d = np.abs(out.cpu().numpy() - ref).max()
+                assert d <= 1e-12 * np.abs(ref).max() + 1e-15, (ls, eps, v)
+            plan.close()
+
+
+@pytest.mark.parametrize("ls", [(0, 0, 0, 0), (1, 0, 1, 0), (2, 1, 1, 1), (2, 1, 2, 2), (3, 2, 2, 2), (3, 3, 3, 3)])
+def test_derivative_roots_at_the_end_of_the_table(ls):
+    """First derivatives on both sides of the table's end of their order (one angular momentum more than
+    the block's): minus the block's derivative by the shell's centre, from the oracle by differences."""
+    import cintx_b200 as cx
+    from oracle import Restatement
+    xmax = XMAX[(sum(ls) + 1) // 2 + 1]
+    q = np.array([[0, 1, 2, 3]], dtype=np.int32)
+    orc = Restatement()
+    h = 1e-2
+    for eps in (-1e-3, -2.0 ** -20 / xmax, -1e-9, 0.0, 1e-9, 1e-3):
+        x = xmax * (1.0 + eps)
+        f = {k: orc.int2e_batch(q, two_centres(ls, x, k * h), sph=True)[0] for k in (-3, -2, -1, 1, 2, 3)}
+        ref = -(45 * (f[1] - f[-1]) - 9 * (f[2] - f[-2]) + (f[3] - f[-3])) / (60 * h)
+        mol = two_centres(ls, x)
+        got, _ = cx.int2e_ip1_sph(q[0], mol.atm, mol.bas, mol.env)
+        dz = got.reshape(3, -1)[2]
+        # sixth-order differences: h^6 / 140 of the seventh derivative (up to some 10^5 in units of a^(7/2)
+        # for f shells), and 1e-14 / h of rounding; a root out of a wrong interval is off by its whole value
+        assert np.abs(dz - ref).max() <= 1e-7 * max(np.abs(ref).max(), np.abs(f[1]).max()), (ls, eps)
+
+
+@pytest.mark.parametrize("sph", [True, False])
+def test_lists_of_generally_contracted_shells_in_any_order(sph):
+    """Every tuple of eight shells of one to two contractions: the blocks of a class come in all index
+    orders, with extents that count the contractions."""
+    import os
+
+    import cintx_b200 as cx
+    import torch
+    from conftest import ROOT
+    from oracle import Restatement
+    g = np.load(os.path.join(ROOT, "tests", "golden", "libcint_ctr2.npz"))
+    mol = M.Molecule("ctr2", g["atm"], g["bas"], g["env"], np.zeros((2, 3)))
+    q = np.stack(np.meshgrid(*[np.arange(mol.nbas)] * 4, indexing="ij"), axis=-1).reshape(-1, 4).astype(np.int32)
+    with cx.Optimizer(mol.atm, mol.bas, mol.env) as opt:
+        plan = cx.Plan.shells(opt, cx.INT2E, q, sph=sph)
+        out = torch.full((plan.stats.nintegrals,), np.nan, dtype=torch.float64, device="cuda")
+        plan.execute(out.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        got = out.cpu().numpy()
+        plan.close()
+    ref, _ = Restatement().int2e_batch(q, mol, sph=sph)
+    agree(got, ref)
 
 
 @pytest.mark.parametrize("sph", [True, False])

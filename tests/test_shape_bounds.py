@@ -31,6 +31,10 @@ def test_every_compiled_launch_shape_keeps_its_indexes_in_bounds(tmp_path):
         assert block <= 1024 and smem <= 227 * 1024
         if glob:  # classes whose transform buffers live in global scratch: one group per block
             assert q == 1
+    # split teams: of 2 groups up to the block's, one-lane ones of at most a warp or the whole block
+    teams = {(r[4], r[5], r[6]) for r in rows if r[4] == "split"}
+    assert {("split", "128", "1"), ("split", "32", "1"), ("split", "2", "64")} <= teams
+    assert ("split", "64", "1") not in teams
     # the sliced and split-transfer cooperative shapes exist where the autotuner can pick them
     assert any(r[4] == "sph" and r[5] == "9" for r in rows)
     for v in ("10", "11"):
