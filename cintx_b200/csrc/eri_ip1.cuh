@@ -94,7 +94,7 @@ __host__ __device__ constexpr int ip1_shape_violation() {
   // the 16-byte column loads: even table sizes behind 2*NR doubles of roots in 16-byte groups
   if (SH::S > 1 && SH::NI % 2 == 0 && (SH::GSZ % 2 != 0 || SH::GROUP_DOUBLES % 2 != 0)) return 11;
   // team barriers of more than a warp and less than the block are named 1 + team: their groups have at
-  // most 32 lanes (no named group barrier), and there are at most 7 of them in 512 threads
+  // most 32 lanes (no named group barrier), and blocks of several groups have at most 128 threads, so two teams
   if (SH::S > 32 && SH::Q > 2) return 12;
   return 0;
 }
@@ -422,7 +422,7 @@ struct Ip1Args {
   cudaStream_t stream;
   int nsplit;       // groups sharing a quartet (power of two)
   int chain;        // kChainPrev, kChainNext (chain.cuh)
-  int* shape;       // not null: launch nothing, write {lanes per group, most groups per quartet, groups per block}
+  int* shape;       // not null: launch nothing, write {lanes per group, most groups per quartet}
 };
 
 template <int LI, int LJ, int LK, int LL, bool SPH>
@@ -431,7 +431,6 @@ cudaError_t launch_ip1(const Ip1Args& a) {
   if (a.shape) {
     a.shape[0] = SH::S;
     a.shape[1] = SH::SPLIT_MAX;
-    a.shape[2] = SH::Q;
     return cudaSuccess;
   }
   if (a.nsplit < 1 || a.nsplit > SH::SPLIT_MAX || (a.nsplit & (a.nsplit - 1)) != 0) return cudaErrorInvalidValue;

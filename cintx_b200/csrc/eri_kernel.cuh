@@ -47,8 +47,6 @@ __host__ __device__ constexpr int binom(int n, int k) {
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 __host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
 
-// Threads per quartet: smallest power of two keeping <= 24 accumulators per lane, capped by
-// the tuple count and by 256.
 // Lanes per quartet: the fewest (a power of two, at most twice the (j,k,l) tuple count) that
 // keep a lane's cartesian accumulators within `acc` doubles.
 __host__ __device__ constexpr int pick_threads(int li, int lj, int lk, int ll, int acc = 24) {
@@ -606,8 +604,8 @@ __global__ void __launch_bounds__(EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SL
                                   EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>::MINB)
     eri4c_kernel(const QuartetRec* __restrict__ recs, int nrec, const ShellPair* __restrict__ pairs,
                  const PrimPair* __restrict__ prims, double* __restrict__ out,
-                 const __grid_constant__ StrideSet sts, double expcutoff, const __grid_constant__ RysTable rys, double* __restrict__ gscratch,
-                 double prim_eps, const double* __restrict__ rootbuf, const long long* __restrict__ rootbase,
+                 const __grid_constant__ StrideSet sts, double expcutoff, const __grid_constant__ RysTable rys,
+                 double* __restrict__ gscratch, double prim_eps, const double* __restrict__ rootbuf, const long long* __restrict__ rootbase,
                  int nsplit, int chain, int nblocks) {
   if (chain_begin(chain, nblocks)) return;
   using SH = EriShape<LI, LJ, LK, LL, SPH, R, ACC, REGS, SLICE, ROLL, PASSES>;

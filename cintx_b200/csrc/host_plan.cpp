@@ -29,9 +29,6 @@
 #include "host_internal.h"
 
 namespace cintx {
-cudaError_t launch_gen_tile(const int* rows, const int* cols, const long long* row_prefix, int nrows,
-                            long long t0, long long t1, long long nout, long long out_base, QuartetRec* recs,
-                            cudaStream_t stream);
 cudaError_t launch_gen_ranges(const GenRange* ranges, int nranges, long long rbegin, long long rend, QuartetRec* recs,
                               cudaStream_t stream);
 cudaError_t launch_prim_x(const QuartetRec* recs, long long nrec, const ShellPair* pairs, const PrimPair* prims,
@@ -601,37 +598,19 @@ static bool segment_scratch(const CintxPlan* p, const Segment& sg) {
 static int run_segment(CintxPlan* p, const Segment& sg, double* out_dev, cudaStream_t stream, DeviceState* ds,
                        ThreadScratch* ts, bool gen, int chain = 0) {
   const Opt* o = p->opt;
-  const QuartetRec* recs;
-  long long nrec;
-  if (sg.tile == -2) {
-    if (gen) {
-      const int rc = gen_records(p, &sg, &sg + 1, stream, ts);
-      if (rc) return rc;
-    }
-    recs = p->d_recs + sg.rec0;
-    nrec = sg.nrec;
-  } else if (sg.tile < 0) {
-    recs = p->d_recs + sg.rec0;
-    nrec = sg.nrec;
-  } else {
-    const Tile& t = p->tiles[sg.tile];
-    QuartetRec* dst = p->d_recs + sg.rec0;
-    cudaError_t e = launch_gen_tile(t.d_rows, t.d_cols, t.d_prefix, (int)t.rows.size(), sg.t0, sg.t1, sg.nout, 0,
-                                    dst, stream);
-    if (e != cudaSuccess) {
-      set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("quartet generation failed: ") + cudaGetErrorString(e));
-      return CINTX_STATUS_EXECUTION_FAILED;
-    }
-    ts->launches++;
-    recs = dst;
-    nrec = sg.t1 - sg.t0;
+  if (gen) {
+    const int rc = gen_records(p, &sg, &sg + 1, stream, ts);
+    if (rc) return rc;
   }
+  const QuartetRec* recs = p->d_recs + sg.rec0;
+  const long long nrec = sg.nrec;
+  const StrideSet st = sg.strides >= 0 ? p->stride_sets[sg.strides] : one_stride(sg.st);
   // the kernels take an int count; split very large segments
   for (long long r0 = 0; r0 < nrec; r0 += 1LL << 30) {
     const int nr = (int)std::min<long long>(nrec - r0, 1LL << 30);
     const bool rb = p->d_rootbuf && sg.tile == -1;  // learned roots: explicit plans only
     cudaError_t e = launch_class(sg.li, sg.lj, sg.lk, sg.ll, p->sph, recs + r0, nr, o->d_pairs, o->d_prims,
-                                 out_dev + sg.out_off, sg.strides >= 0 ? p->stride_sets[sg.strides] : one_stride(sg.st), sg.expcutoff, ds->rys, stream, sg.fp32, sg.prim_eps,
+                                 out_dev + sg.out_off, st, sg.expcutoff, ds->rys, stream, sg.fp32, sg.prim_eps,
                                  sg.variant, rb ? p->d_rootbuf : nullptr, rb ? p->d_rootbase + sg.rec0 + r0 : nullptr,
                                  sg.groups(), chain);
     if (e != cudaSuccess) {

@@ -227,7 +227,7 @@ int ip1_launch(const Ip1Work& W, bool sph, int nsh, const Basis& B, char* dev, c
     const Ip1Work::Key& k = kv.first;
     const std::vector<QuartetRec>& recs = kv.second.recs;
     QuartetRec* dst = reinterpret_cast<QuartetRec*>(host + o_recs) + r0;
-    int shape[3];
+    int shape[2];
     Ip1Args qa{};
     qa.shape = shape;
     if (dispatch_ip1(k.li, k.lj, k.lk, k.ll, sph, qa) != cudaSuccess) {

@@ -1,9 +1,8 @@
 // Device-side quartet generation for screened plans.
 //
 // A tile (A, B) of a screened plan pairs every shell pair p of pair type A (sorted by
-// decreasing Schwarz factor) with the first count[p] pairs of type B.  Quartets are numbered
-// row-major; row_prefix[r] is the first quartet index of row r.  One thread per quartet finds
-// its row by binary search and writes the record; out offsets are consecutive blocks.
+// decreasing Schwarz factor) with a run of the pairs of type B.  Quartets are numbered row-major;
+// prefix[r] is the first quartet index of row r.  Out offsets are consecutive blocks.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -12,47 +11,17 @@
 #include "chain.cuh"
 #include "common.h"
 
-__global__ void gen_tile_quartets(const int* __restrict__ rows, const int* __restrict__ cols,
-                                  const long long* __restrict__ row_prefix, int nrows, long long t0,
-                                  long long t1, long long nout, long long out_base,
-                                  QuartetRec* __restrict__ recs) {
-  for (long long t = t0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; t < t1;
-       t += (long long)gridDim.x * blockDim.x) {
-    int lo = 0, hi = nrows - 1;  // last row with row_prefix[row] <= t
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (row_prefix[mid] <= t) lo = mid;
-      else hi = mid - 1;
-    }
-    QuartetRec r;
-    r.pij = rows[lo];
-    r.pkl = cols[t - row_prefix[lo]];
-    r.out = out_base + (t - t0) * nout;
-    recs[t - t0] = r;
-  }
-}
-
 namespace cintx {
-cudaError_t launch_gen_tile(const int* rows, const int* cols, const long long* row_prefix, int nrows,
-                            long long t0, long long t1, long long nout, long long out_base, QuartetRec* recs,
-                            cudaStream_t stream) {
-  const long long n = t1 - t0;
-  if (n <= 0) return cudaSuccess;
-  long long blocks = (n + 255) / 256;
-  if (blocks > 65535) blocks = 65535;
-  gen_tile_quartets<<<(unsigned)blocks, 256, 0, stream>>>(rows, cols, row_prefix, nrows, t0, t1, nout, out_base,
-                                                           recs);
-  return cudaGetLastError();
+int device_sm_count();
 }
-}  // namespace cintx
 
 // Multi-range generation: one launch fills records [rbegin, rend) of a chunk: of the whole chunk when
 // it is run as one, of a single class segment when that is run alone.  ranges[] are the tile ranges that
 // hold them, ordered by rec_off (a range's first record); record r belongs to the last range whose
 // rec_off <= r.
 //
-// A warp writes `run` consecutive records (kGenRun, fewer where that would leave the chip idle), 32 at a time.  Its lanes search the range and the row of
-// the warp's first record together (the same addresses for all lanes); a record a few places on is then
+// A warp writes `run` consecutive records (kGenRun, fewer where that would leave the chip idle), 32 at a
+// time.  Its lanes search the range and the row of the warp's first record together (the same addresses for all lanes); a record a few places on is then
 // usually in the same row, and where it is not, every row between holds at least one record, so its row
 // lies within that many rows of the first one's and a short search ends there.  (One full search of
 // both lists per record was bound by the latency of its dependent loads.)  Records of a 40-atom
@@ -118,8 +87,8 @@ __global__ void gen_range_quartets(const GenRange* __restrict__ ranges, int nran
 
 // x = a_ij a_kl / (a_ij + a_kl) |P - Q|^2 of every primitive quartet (b over the (kl) pair's
 // primitives, a over the (ij) pair's, the ERI kernels' loop order) of nrec records, written at
-// xout[pbase[r] + b * npij + a]; the same expression as the kernels, so the roots computed from
-// it are the ones those kernels would evaluate.
+// xout[pbase[r] + b * npij + a].  The kernels' own table roots are evaluated at an x that differs from
+// this one by rounding (rys_point).
 __global__ void prim_x_kernel(const QuartetRec* __restrict__ recs, long long nrec, const ShellPair* __restrict__ pairs,
                               const PrimPair* __restrict__ prims, const long long* __restrict__ pbase,
                               double* __restrict__ xout) {
@@ -256,8 +225,8 @@ __global__ void jk_contract_kernel(const QuartetRec* __restrict__ recs, long lon
 // s1 of 14 (1.9 GB, 254 of it the clearing) 980 -> 947.
 template <int MODE>
 __global__ void scatter_ao_kernel(const QuartetRec* __restrict__ recs, long long nrec, const int2* __restrict__ pao,
-                                  const double* __restrict__ out, double* __restrict__ eri, long long nao, SmallDiv ni, SmallDiv nj, SmallDiv nk,
-                                  SmallDiv nl, int G, int chain, int nblocks) {
+                                  const double* __restrict__ out, double* __restrict__ eri, long long nao,
+                                  SmallDiv ni, SmallDiv nj, SmallDiv nk, SmallDiv nl, int G, int chain, int nblocks) {
   if (chain_begin(chain, nblocks)) return;
   const int g = threadIdx.x & (G - 1);
   const long long npair = nao * (nao + 1) / 2, n2 = nao * nao;
@@ -343,8 +312,9 @@ __global__ void scatter_ao_kernel(const QuartetRec* __restrict__ recs, long long
 // kJkRun, fewer where the records would not give every resident warp work) and adds A[i,j] once per run
 // and pair.
 //
-// Bound: the atomics, about (nk + nl)(ni + nj) + nk nl per quartet, at the L2's rate.  J+K of 120
-// s/p/d/f atoms (5.7e9 integrals): 139 ms of contraction with six passes over each block, 68 ms so.
+// Bound: instructions and the gathers of the density; the atomics, about (nk + nl)(ni + nj) + nk nl per
+// quartet, are not (leaving them all out: 2%).  J+K of 120 s/p/d/f atoms (5.7e9 integrals): 139 ms of
+// contraction with six passes over each block, 68 ms so, 48 with jk_contract_thread_kernel and the rest.
 constexpr int kJkRun = 16;
 constexpr int kJkWarps = 4;
 
@@ -684,11 +654,11 @@ static cudaError_t launch_jk_group(const QuartetRec* recs, long long nrec, const
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) attr_done[dev] = 1;
   }
-  const long long resident = 148LL * 16 * (32 / G);  // groups, 16 warps per SM
+  const long long resident = (long long)device_sm_count() * 16 * (32 / G);  // groups, 16 warps per SM
   const int run = (int)std::max(1LL, std::min<long long>(kJkRun, nrec / (2 * resident)));
   const long long per_block = 32LL * kJkWarps / G * run;
   long long blocks = (nrec + per_block - 1) / per_block;
-  if (blocks > 148LL * 64) blocks = 148LL * 64;
+  if (blocks > (long long)device_sm_count() * 64) blocks = (long long)device_sm_count() * 64;
   return chain_launch(kern, (unsigned)blocks, 32 * kJkWarps, smem, stream, chain, recs, nrec, pao, out, dm, nao, A, B,
                       small_divisor(ni), small_divisor(nj), G, run);
 }
@@ -697,7 +667,7 @@ template <int NI, int NK>
 static cudaError_t launch_jk_thread(const QuartetRec* recs, long long nrec, const int2* pao, const double* out,
                                     const double* dm, int nao, double* A, double* B, cudaStream_t stream, int nj,
                                     int chain) {
-  const long long blocks = std::min((nrec + 127) / 128, 148LL * 64);
+  const long long blocks = std::min((nrec + 127) / 128, (long long)device_sm_count() * 64);
   return chain_launch(jk_contract_thread_kernel<NI, NK>, (unsigned)blocks, 128, 0, stream, chain, recs, nrec, pao, out,
                       dm, nao, A, B, nj);
 }
@@ -718,7 +688,7 @@ cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int
 #define CINTX_JK(K, L) \
   if (nk == K && nl == L) return launch_jk_group<K, L>(recs, nrec, pao, out, dm, nao, A, B, stream, ni, nj, chain);
   if (jk_group_smem(ni * nj, nk, nl) <= kJkSmem) {
-    CINTX_JK(1, 1) CINTX_JK(3, 1) CINTX_JK(3, 3)  // (1, 1) and (3, 1): cartesian g first shells
+    CINTX_JK(1, 1) CINTX_JK(3, 1) CINTX_JK(3, 3)  // (1, 1): cartesian f and g first shells, (3, 1): spherical g too
     CINTX_JK(5, 1) CINTX_JK(5, 3) CINTX_JK(5, 5)
     CINTX_JK(6, 1) CINTX_JK(6, 3) CINTX_JK(6, 6)
     CINTX_JK(7, 1) CINTX_JK(7, 3) CINTX_JK(7, 5) CINTX_JK(7, 7)
@@ -727,7 +697,7 @@ cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int
   }
 #undef CINTX_JK
   long long blocks = (nrec * 32 + 255) / 256;
-  if (blocks > 148LL * 64) blocks = 148LL * 64;
+  if (blocks > (long long)device_sm_count() * 64) blocks = (long long)device_sm_count() * 64;
   return chain_launch(jk_contract_kernel, (unsigned)blocks, 256, 0, stream, chain, recs, nrec, pao, out, dm, nao, A, B,
                       ni, nj, nk, nl);
 }
@@ -739,7 +709,7 @@ cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2
   int G = 1;
   while (G < 32 && G < ni * nj * nk * nl) G *= 2;
   long long blocks = (nrec * G + 255) / 256;
-  if (blocks > 148LL * 64) blocks = 148LL * 64;
+  if (blocks > (long long)device_sm_count() * 64) blocks = (long long)device_sm_count() * 64;
   auto kern = mode == 1 ? scatter_ao_kernel<1> : (mode == 4 ? scatter_ao_kernel<4> : scatter_ao_kernel<8>);
   return chain_launch(kern, (unsigned)blocks, 256, 0, stream, chain, recs, nrec, pao, out, eri, nao, small_divisor(ni),
                       small_divisor(nj), small_divisor(nk), small_divisor(nl), G);
@@ -748,7 +718,7 @@ cudaError_t launch_scatter_ao(const QuartetRec* recs, long long nrec, const int2
 cudaError_t launch_symmetrize(const double* X, double* M, int n, cudaStream_t stream) {
   const long long total = (long long)n * n;
   long long blocks = (total + 255) / 256;
-  if (blocks > 148LL * 32) blocks = 148LL * 32;
+  if (blocks > (long long)device_sm_count() * 32) blocks = (long long)device_sm_count() * 32;
   if (total > 0) symmetrize_kernel<<<(unsigned)blocks, 256, 0, stream>>>(X, M, n);
   return cudaGetLastError();
 }
@@ -757,7 +727,7 @@ cudaError_t launch_gen_ranges(const GenRange* ranges, int nranges, long long rbe
                               cudaStream_t stream) {
   const long long nrec = rend - rbegin;
   if (nrec <= 0) return cudaSuccess;
-  const int run = 32 * (int)std::max(1LL, std::min<long long>(kGenRun / 32, nrec / (148 * 64 * 32)));
+  const int run = 32 * (int)std::max(1LL, std::min<long long>(kGenRun / 32, nrec / (device_sm_count() * 64LL * 32)));
   long long blocks = (nrec + 8 * run - 1) / (8 * run);  // 8 warps per block
   if (blocks > 65535) blocks = 65535;
   gen_range_quartets<<<(unsigned)blocks, 256, 0, stream>>>(ranges, nranges, rbegin, rend, recs, run);
