@@ -1051,7 +1051,7 @@ def our_arm(args):
         line["decomposition"] = {
             "plain_fp64": pv, "fp64_autotuned_shapes": sv, "tuned": value,
             "autotuner_factor": sv / pv, "primitive_screening_factor": value / sv,
-            "what": "plain = default shapes, libcint screening; fp64_autotuned_shapes = the tuned plan's launch shapes "
+            "what": "plain = untuned plan (launch shapes by rule), libcint screening; fp64_autotuned_shapes = the tuned plan's launch shapes "
                     "with no primitive screening and no FP32; tuned = this line's value (autotuned shapes + primitive "
                     "Schwarz screening within %g per integral)" % args.prim_budget}
     if "north_star" in extra:
