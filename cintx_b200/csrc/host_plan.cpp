@@ -1806,8 +1806,9 @@ int diag_schwarz_2e(Opt* o, double ecut, std::vector<double>& Q, int np) {
           for (int part = 0; part < 2 && ok; ++part) {
             const long long q0 = part ? rs : r0, q1 = part ? seg_end[g] : rs;
             if (q1 <= q0) continue;
-            ok = launch_class(la, lb, la, lb, true, d_recs + q0, (int)(q1 - q0), o->d_pairs, o->d_prims, d_out, one_stride(st),
-                              ecut, ds->rys, ts->stream, false, 0.0, default_variant(la, lb, la, lb, mean_np[seg_cls[g]]), nullptr, nullptr,
+            ok = launch_class(la, lb, la, lb, true, d_recs + q0, (int)(q1 - q0), o->d_pairs, o->d_prims, d_out,
+                              one_stride(st), ecut, ds->rys, ts->stream, false, 0.0,
+                              default_variant(la, lb, la, lb, mean_np[seg_cls[g]]), nullptr, nullptr,
                               part ? 1 : ps.ns) ==
                  cudaSuccess;
             ts->launches++;

@@ -252,8 +252,8 @@ extern "C" int cintx_int2e_noalloc(double* out_dev, const int* shls, int64_t n, 
     st.s3 = k.s3;
     for (size_t a = 0; a < L.second.second; a += (size_t)1 << 30) {
       const int nr = (int)std::min<size_t>(L.second.second - a, (size_t)1 << 30);
-      e = launch_class(k.li, k.lj, k.lk, k.ll, sp, drecs + L.second.first + a, nr, dpairs, dprims, out_dev, one_stride(st), cutoff,
-                       nd->rys, s);
+      e = launch_class(k.li, k.lj, k.lk, k.ll, sp, drecs + L.second.first + a, nr, dpairs, dprims, out_dev,
+                       one_stride(st), cutoff, nd->rys, s);
       if (e != cudaSuccess) {
         set_error(CINTX_STATUS_EXECUTION_FAILED, std::string("kernel launch failed: ") + cudaGetErrorString(e));
         return CINTX_STATUS_EXECUTION_FAILED;

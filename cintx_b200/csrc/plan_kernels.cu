@@ -21,11 +21,12 @@ int device_sm_count();
 // rec_off <= r.
 //
 // A warp writes `run` consecutive records (kGenRun, fewer where that would leave the chip idle), 32 at a
-// time.  Its lanes search the range and the row of the warp's first record together (the same addresses for all lanes); a record a few places on is then
-// usually in the same row, and where it is not, every row between holds at least one record, so its row
-// lies within that many rows of the first one's and a short search ends there.  (One full search of
-// both lists per record was bound by the latency of its dependent loads.)  Records of a 40-atom
-// s/p/d sweep: 362 us in a launch per class with one search per record, 80 us so; of 12 atoms 157 and 11 us.
+// time.  Its lanes search the range and the row of the warp's first record together (the same addresses for
+// all lanes); a record a few places on is then usually in the same row, and where it is not, every row between
+// holds at least one record, so its row lies within that many rows of the first one's and a short search ends
+// there.  (One full search of both lists per record was bound by the latency of its dependent loads.)
+// Records of a 40-atom s/p/d sweep: 362 us in a launch per class with one search per record, 80 us so; of 12
+// atoms 157 and 11 us.
 constexpr int kGenRun = 256;
 
 __global__ void gen_range_quartets(const GenRange* __restrict__ ranges, int nranges, long long rbegin,
@@ -681,7 +682,8 @@ cudaError_t launch_jk_contract(const QuartetRec* recs, long long nrec, const int
                                int ni, int nj, int nk, int nl, int chain) {
   if (nrec <= 0) return cudaSuccess;
 #define CINTX_JK_THREAD(I, K) \
-  if (ni == I && nk == K && nl == 1) return launch_jk_thread<I, K>(recs, nrec, pao, out, dm, nao, A, B, stream, nj, chain);
+  if (ni == I && nk == K && nl == 1)  \
+    return launch_jk_thread<I, K>(recs, nrec, pao, out, dm, nao, A, B, stream, nj, chain);
   CINTX_JK_THREAD(1, 1) CINTX_JK_THREAD(3, 1) CINTX_JK_THREAD(5, 1) CINTX_JK_THREAD(6, 1) CINTX_JK_THREAD(7, 1)
   CINTX_JK_THREAD(9, 1) CINTX_JK_THREAD(3, 3) CINTX_JK_THREAD(5, 3) CINTX_JK_THREAD(6, 3) CINTX_JK_THREAD(7, 3)
 #undef CINTX_JK_THREAD
